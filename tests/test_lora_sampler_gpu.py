@@ -129,6 +129,32 @@ def test_paged_decode(E):
     assert rel(o, r) < 6e-3
 
 
+@pytest.mark.parametrize('hq,hkv,D,bs,cap', [(32, 8, 128, 16, 8), (16, 1, 128, 16, 256), (40, 4, 64, 8, 700), (12, 3, 64, 24, 40), (8, 1, 128, 1, 600), (6, 2, 64, 24, 40)])
+def test_paged_decode_splits(E, hq, hkv, D, bs, cap):
+    """Contexts around tile (16), warp and cluster boundaries, tables wide enough for one to eight CTAs per key head, groups of 3 (the vector kernel) to 16 heads."""
+    from twinkle_b200 import ops
+    torch.manual_seed(hq + D)
+    lens = [n for n in (0, 1, 15, 16, 17, 63, 64, 65, 127, 128, 513, 1025, 2000) if n <= bs * cap]
+    need = [(n + bs - 1) // bs for n in lens]
+    nblocks = sum(need) + 1
+    kc, vc = (torch.randn(nblocks, bs, hkv, D, device='cuda').bfloat16() for _ in range(2))
+    kc[0], vc[0] = float('nan'), float('nan')                       # nobody's block
+    perm, tables, used = (torch.randperm(nblocks - 1) + 1).int(), torch.zeros(len(lens), cap, dtype=torch.int32), 0
+    for i, nb in enumerate(need):
+        tables[i, :nb] = perm[used:used + nb]
+        used += nb
+    q = torch.randn(len(lens), hq, D, device='cuda').bfloat16()
+    o = ops.paged_attention_decode(q, kc, vc, tables.cuda(), torch.tensor(lens, dtype=torch.int32, device='cuda')).double()
+    for i, (n, nb) in enumerate(zip(lens, need)):
+        if n == 0:
+            assert not o[i].any()
+            continue
+        at = tables[i, :nb].long().cuda()
+        k, v = (c[at].flatten(0, 1)[:n].double().repeat_interleave(hq // hkv, 1) for c in (kc, vc))
+        w = torch.softmax(torch.einsum('hd,nhd->hn', q[i].double(), k) * D ** -0.5, -1)
+        assert rel(o[i], torch.einsum('hn,nhd->hd', w, v)) < 2.5e-3, n      # rounding of the result to bf16: 2^-9 = 2e-3 at most
+
+
 def test_router(E):
     from twinkle_b200 import ops
     torch.manual_seed(4)

@@ -1,13 +1,14 @@
 // Sampler kernels: paged-KV decode attention (one query token per sequence, GQA), token sampling
 // (temperature / top-k / top-p via threshold bisection + Gumbel-max, log-prob of the processed
 // distribution), and the MoE router (fp32 softmax + top-k + renormalisation + expert histogram).
-// All three are bandwidth / latency bound; none needs tensor cores.
+// All three are bandwidth / latency bound.  Groups of four query heads and more decode on the tensor cores (paged_decode.cu).
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/types.h>
 
 #include "common.cuh"
 #include "host.h"
+#include "paged_decode.h"
 #include "scores.cuh"
 
 namespace tk {
@@ -244,6 +245,14 @@ torch::Tensor paged_attn_decode(const torch::Tensor& q, const torch::Tensor& kc,
   const float sl2 = static_cast<float>(scale * 1.4426950408889634);
   auto stream = at::cuda::getCurrentCUDAStream();
   auto run = [&](auto tag, auto terms) { launch_paged_decode<decltype(tag), decltype(terms)::value>(q, kc, vc, tables, seq_lens, out, sl2, x, stream); };
+  if (st == torch::kBFloat16 && !x.terms.used) {
+    const PagedDecode p{q.data_ptr(), kc.data_ptr(), vc.data_ptr(), tables.data_ptr<int>(), seq_lens.data_ptr<int>(), out.data_ptr(), x.sinks, x.gate, static_cast<int>(q.size(1)),
+                        static_cast<int>(kc.size(2)), static_cast<int>(q.size(1) / kc.size(2)), static_cast<int>(kc.size(1)), static_cast<int>(tables.size(1)), x.window, x.chunk, sl2};
+    if (paged_decode_mma(p, q.size(0), q.size(2), vc.size(3), stream)) {
+      count_launch();
+      return out;
+    }
+  }
   if (st == torch::kBFloat16) {
     if (x.terms.used) run(bf16{}, std::true_type{}); else run(bf16{}, std::false_type{});
   } else {
