@@ -345,3 +345,38 @@ def test_decode_cuda_graph_matches_eager(E):
     for (t1, l1), (t0, l0) in zip(outs[True], outs[False]):
         assert t1 == t0
         assert max(abs(a - b) for a, b in zip(l1, l0)) < 1e-3
+
+
+@pytest.mark.parametrize('V', [1, 7, 33, 4099, 32000, 151936, 400001])
+@pytest.mark.parametrize('kind', ['flat', 'normal', 'peaked', 'masked'])
+def test_sampling_thresholds(E, V, kind):
+    """What is kept, from sorted fp64 probabilities, for rows that leave parts of a cluster empty, fill its shared memory, exceed it (400001), whose
+    bracket holds everything (flat) or nothing but the largest (peaked), and with tokens ruled out."""
+    from twinkle_b200 import ops
+    g = torch.Generator(device='cuda').manual_seed(V)
+    x = torch.randn(6, V, device='cuda', generator=g)
+    if kind == 'flat':
+        x *= 1e-3
+    elif kind == 'peaked':
+        x[:, V // 2] += 60.0
+    elif kind == 'masked':
+        x *= 3
+        x[:, 1:][torch.rand(6, V - 1, device='cuda', generator=g) < 0.7] = float('-inf')
+    seeds = torch.arange(6, device='cuda')
+    for temp, k, p in [(1.0, -1, 0.9), (0.7, 5, 1.0), (1.0, 50, 0.8), (1.3, -1, 1.0), (1.0, -1, 0.2)]:
+        tok, lp = ops.sample_tokens(x, temp, k, p, seeds=seeds)
+        prob = torch.softmax(x.double() / temp, -1)
+        top, _ = prob.sort(-1, descending=True)
+        tau = torch.zeros(6, dtype=torch.float64, device='cuda')
+        if 0 < k < V:
+            tau = torch.maximum(tau, top[:, k - 1])
+        if p < 1:
+            tau = torch.maximum(tau, top.gather(1, (top.cumsum(-1) < p).sum(-1, keepdim=True).clamp_max(V - 1))[:, 0])
+        mine = prob.gather(1, tok[:, None])[:, 0]
+        step = top[:, 0] * 2.0 ** -32 + tau * 1e-5            # resolution of the search, and of fp32 probabilities
+        assert (mine >= tau - step).all()
+        low, high = (torch.where(prob >= (tau + s * step)[:, None], prob, 0).sum(-1) for s in (1, -1))     # mass kept, but for the tokens at the border
+        want = mine.log()
+        assert (lp >= want - high.log() - 2e-5).all() and (lp <= want - torch.maximum(low, top[:, 0]).log() + 2e-5).all()
+        again, lp2 = ops.sample_tokens(x, temp, k, p, seeds=seeds)
+        assert torch.equal(tok, again) and torch.equal(lp, lp2)

@@ -1,7 +1,5 @@
-// Sampler kernels: paged-KV decode attention (one query token per sequence, GQA), token sampling
-// (temperature / top-k / top-p via threshold bisection + Gumbel-max, log-prob of the processed
-// distribution), and the MoE router (fp32 softmax + top-k + renormalisation + expert histogram).
-// All three are bandwidth / latency bound.  Groups of four query heads and more decode on the tensor cores (paged_decode.cu).
+// Sampler kernels: paged-KV decode attention (one query token per sequence, GQA) and the MoE router (fp32 softmax + top-k +
+// renormalisation + expert histogram).  Both are bandwidth / latency bound.  Groups of four query heads and more decode on the tensor cores (paged_decode.cu).
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/types.h>
@@ -261,144 +259,6 @@ torch::Tensor paged_attn_decode(const torch::Tensor& q, const torch::Tensor& kc,
   count_launch();
   TK_CUDA_CHECK(cudaGetLastError());
   return out;
-}
-
-// -------------------------------------------------------------------- sampling
-__device__ __forceinline__ float block_reduce(float v, bool is_max, float* sh) {
-  v = is_max ? warp_max(v) : warp_sum(v);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) sh[warp] = v;
-  __syncthreads();
-  const int nw = blockDim.x >> 5;
-  float r = lane < nw ? sh[lane] : (is_max ? -INFINITY : 0.f);
-  r = is_max ? warp_max(r) : warp_sum(r);
-  return __shfl_sync(0xffffffffu, r, 0);
-}
-__device__ __forceinline__ uint32_t mix32(uint64_t x) {
-  x ^= x >> 33; x *= 0xff51afd7ed558ccdull; x ^= x >> 33; x *= 0xc4ceb9fe1a85ec53ull; x ^= x >> 33;
-  return static_cast<uint32_t>(x);
-}
-
-// One CTA per row.  kept set = {p ≥ τ}: τ from bisection so that |kept| ≤ top_k-ish and mass(kept) ≥ top_p
-// (the smallest such set up to ties).  Token = argmax over kept of (x/T + Gumbel noise).
-__global__ void __launch_bounds__(512) sample_kernel(const float* __restrict__ logits, const int64_t* __restrict__ seeds, int64_t* __restrict__ tok,
-                                                      float* __restrict__ logprob, int V, float inv_temp, int top_k, float top_p, int greedy) {
-  __shared__ float sh[32];
-  __shared__ int sh_i[32];
-  const int row = blockIdx.x;
-  const float* x = logits + static_cast<size_t>(row) * V;
-  // max and sum-exp in one pass (online softmax per thread, merged across the block)
-  float mx = -INFINITY, z = 0.f;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    const float y = x[i] * inv_temp;
-    if (y > mx) { z = z * __expf(mx - y) + 1.f; mx = y; } else { z += __expf(y - mx); }
-  }
-  {
-    const float m_all = block_reduce(mx, true, sh);
-    z = block_reduce(z * __expf(mx - m_all), false, sh);
-    mx = m_all;
-  }
-  float tau = 0.f, kept_mass = 1.f;  // threshold on p = e^{x−mx}/z
-  const bool use_k = top_k > 0 && top_k < V, use_p = top_p < 1.f;
-  if (!greedy && (use_k || use_p)) {
-    // τ_k: highest threshold that still keeps ≥ k tokens; τ_p: highest that still keeps mass ≥ top_p; the kept set
-    // respects both limits → τ = max(τ_k, τ_p).  Each pass over the row tests 15 thresholds per search (16-way
-    // narrowing of [lo, hi)), so 8 passes resolve both thresholds to 2⁻³² of the largest probability.
-    constexpr int NT = 15;
-    float lo_k = 0.f, hi_k = 1.f / z, lo_p = 0.f, hi_p = 1.f / z;  // p_max = 1/z
-    const float inv_z = 1.f / z;
-    for (int it = 0; it < 8; ++it) {
-      float ck[NT], cp[NT];
-#pragma unroll
-      for (int j = 0; j < NT; ++j) { ck[j] = 0.f; cp[j] = 0.f; }
-      const float dk = (hi_k - lo_k) * (1.f / 16.f), dp = (hi_p - lo_p) * (1.f / 16.f);
-      for (int i = threadIdx.x; i < V; i += blockDim.x) {
-        const float p = __expf(x[i] * inv_temp - mx) * inv_z;
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-          ck[j] += (p >= lo_k + dk * (j + 1)) ? 1.f : 0.f;
-          cp[j] += (p >= lo_p + dp * (j + 1)) ? p : 0.f;
-        }
-      }
-      int jk = -1, jp = -1;
-#pragma unroll
-      for (int j = 0; j < NT; ++j) {
-        const float a_k = use_k ? block_reduce(ck[j], false, sh) : 0.f;
-        const float a_p = use_p ? block_reduce(cp[j], false, sh) : 0.f;
-        if (a_k >= static_cast<float>(top_k)) jk = j;   // counts and masses fall with j: the last j that passes is the highest
-        if (a_p >= top_p) jp = j;
-      }
-      const float nlo_k = lo_k + dk * (jk + 1), nlo_p = lo_p + dp * (jp + 1);
-      hi_k = (jk == NT - 1) ? hi_k : nlo_k + dk;
-      hi_p = (jp == NT - 1) ? hi_p : nlo_p + dp;
-      lo_k = nlo_k;
-      lo_p = nlo_p;
-    }
-    tau = fmaxf(use_k ? lo_k : 0.f, use_p ? lo_p : 0.f);
-    float mass = 0.f;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-      const float p = __expf(x[i] * inv_temp - mx) * inv_z;
-      if (p >= tau) mass += p;
-    }
-    kept_mass = block_reduce(mass, false, sh);
-  }
-  float best = -INFINITY;
-  int best_i = 0;
-  const uint64_t seed = static_cast<uint64_t>(seeds[row]);
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    const float xs = x[i] * inv_temp;
-    const float p = __expf(xs - mx) / z;
-    if (p < tau) continue;
-    float score = xs;
-    if (!greedy) {
-      const float u = (static_cast<float>(mix32(seed * 0x9E3779B97F4A7C15ull + static_cast<uint64_t>(i))) + 0.5f) * (1.f / 4294967296.f);
-      score += -__logf(-__logf(u));
-    }
-    if (score > best) { best = score; best_i = i; }
-  }
-  // block arg-max
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
-    if (ob > best || (ob == best && oi < best_i)) { best = ob; best_i = oi; }
-  }
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  __syncthreads();
-  if (lane == 0) { sh[warp] = best; sh_i[warp] = best_i; }
-  __syncthreads();
-  if (warp == 0) {
-    best = lane < (blockDim.x >> 5) ? sh[lane] : -INFINITY;
-    best_i = lane < (blockDim.x >> 5) ? sh_i[lane] : 0;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const float ob = __shfl_xor_sync(0xffffffffu, best, o);
-      const int oi = __shfl_xor_sync(0xffffffffu, best_i, o);
-      if (ob > best || (ob == best && oi < best_i)) { best = ob; best_i = oi; }
-    }
-    if (lane == 0) {
-      tok[row] = best_i;
-      logprob[row] = greedy ? 0.f : (x[best_i] * inv_temp - mx - __logf(z) - __logf(kept_mass));
-    }
-  }
-}
-
-std::vector<torch::Tensor> sample_tokens(const torch::Tensor& logits, double temperature, int64_t top_k, double top_p, const torch::Tensor& seeds) {
-  TORCH_CHECK(logits.is_cuda() && logits.scalar_type() == torch::kFloat32 && logits.is_contiguous() && logits.dim() == 2, "logits [B,V] fp32");
-  TORCH_CHECK(seeds.is_cuda() && seeds.scalar_type() == torch::kInt64 && seeds.numel() == logits.size(0), "seeds int64 [B]");
-  c10::cuda::CUDAGuard guard(logits.device());
-  const int B = logits.size(0), V = logits.size(1);
-  auto tok = torch::empty({B}, logits.options().dtype(torch::kInt64));
-  auto lp = torch::empty({B}, logits.options());
-  if (B == 0) return {tok, lp};
-  const bool greedy = temperature <= 0.0;
-  sample_kernel<<<B, 512, 0, at::cuda::getCurrentCUDAStream()>>>(logits.data_ptr<float>(), seeds.data_ptr<int64_t>(), tok.data_ptr<int64_t>(),
-                                                                 lp.data_ptr<float>(), V, greedy ? 1.f : static_cast<float>(1.0 / temperature),
-                                                                 static_cast<int>(top_k), static_cast<float>(top_p), greedy ? 1 : 0);
-  count_launch();
-  TK_CUDA_CHECK(cudaGetLastError());
-  return {tok, lp};
 }
 
 // ---------------------------------------------------------------------- router
