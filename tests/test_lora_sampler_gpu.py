@@ -380,3 +380,33 @@ def test_sampling_thresholds(E, V, kind):
         assert (lp >= want - high.log() - 2e-5).all() and (lp <= want - torch.maximum(low, top[:, 0]).log() + 2e-5).all()
         again, lp2 = ops.sample_tokens(x, temp, k, p, seeds=seeds)
         assert torch.equal(tok, again) and torch.equal(lp, lp2)
+
+
+@pytest.mark.parametrize('M', [1, 7, 8, 9, 120, 127, 128, 129, 300])
+@pytest.mark.parametrize('N,K', [(16, 64), (40, 192), (1000, 320), (1024, 3072), (6144, 1024), (520, 8192), (4096, 12288)])
+def test_gemm_few_rows(E, M, N, K):
+    """Narrow tiles for few rows: the bits of the wide tiles where K is not split, fp64 to the rounding of sums otherwise; ragged rows and columns,
+    strided operands, both result types, accumulation."""
+    g = torch.Generator(device='cuda').manual_seed(M * 7 + N)
+    x = torch.randn(M, K + 64, device='cuda', generator=g).bfloat16()[:, :K]
+    w = torch.randn(N, K, device='cuda', generator=g).bfloat16()
+    want = x.double() @ w.double().t()
+    for dt in (torch.bfloat16, torch.float32):
+        y = E.gemm(x, w, 'nt', None, False, dt)
+        E.set_gemm_pair(0)
+        wide = E.gemm(x, w, 'nt', None, False, dt)
+        E.set_gemm_pair(1)
+        if K < 8192:
+            assert torch.equal(y, wide)
+        # fp32 accumulation of K products of unit variance: K·2^-24 of √K at worst; one rounding to bf16 is 2^-9 of a value
+        bound = K * 2.0 ** -24 * K ** 0.5 * 4 + (want.abs() * 2.0 ** -8 if dt == torch.bfloat16 else 0.0)
+        assert ((y.double() - want).abs() <= bound).all()
+        out = torch.randn(M, N + 8, device='cuda', generator=g).to(dt)
+        before, ref = out.clone(), out.clone()
+        E.gemm(x, w, 'nt', out[:, :N], True)
+        E.set_gemm_pair(0)
+        E.gemm(x, w, 'nt', ref[:, :N], True)
+        E.set_gemm_pair(1)
+        assert torch.equal(out[:, N:], before[:, N:])
+        assert torch.equal(out, ref) if K < 8192 else rel(out, ref) < 4e-3
+    assert E.read_and_clear_error() == 0

@@ -401,7 +401,9 @@ static void check_operand(const torch::Tensor& t, const char* name) {
 bool gemm_pair_launch(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb, void* out, int M, int N, int K, int ldo,
                       bool out_fp32, bool accumulate, cudaStream_t stream);
 
-// 0: single-CTA tiles only; 1: SM-pair kernel (gemm2.cu) for shapes with enough 256x256 tiles to fill the device.
+bool gemm_skinny(const torch::Tensor& a, const torch::Tensor& b, void* out, int M, int N, int K, int ldo, bool out_fp32, bool accumulate, cudaStream_t stream);
+
+// 0: single-CTA tiles only; 1: narrow tiles (gemm_skinny.cu) for few rows, SM-pair kernel (gemm2.cu) for shapes with enough 256x256 tiles to fill the device.
 static int g_pair_mode = [] {
   const char* e = getenv("TK_GEMM_PAIR");
   return e ? atoi(e) : 1;
@@ -434,6 +436,9 @@ torch::Tensor gemm(const torch::Tensor& a, const torch::Tensor& b, const std::st
               "out rows must be 16-byte aligned");
   if (M == 0 || N == 0) return out;
   if (K == 0) { if (!accumulate) out.zero_(); return out; }
+  if (g_pair_mode && layout == "nt" &&
+      gemm_skinny(a, b, out.data_ptr(), M, N, K, static_cast<int>(out.stride(0)), fp32, accumulate, at::cuda::getCurrentCUDAStream()))
+    return out;
   if (g_pair_mode && ((M + 255) / 256) * ((N + 255) / 256) >= num_sms() / 2) {
     CUtensorMap pa = a_mn ? make_tmap_2d(a.data_ptr(), a.size(1), a.size(0), a.stride(0), 64, BK)
                           : make_tmap_2d(a.data_ptr(), a.size(1), a.size(0), a.stride(0), BK, 128);
