@@ -410,3 +410,33 @@ def test_gemm_few_rows(E, M, N, K):
         assert torch.equal(out[:, N:], before[:, N:])
         assert torch.equal(out, ref) if K < 8192 else rel(out, ref) < 4e-3
     assert E.read_and_clear_error() == 0
+
+
+@pytest.mark.parametrize('hq,hkv', [(4, 4), (8, 1), (6, 2), (16, 4), (64, 32)])
+@pytest.mark.parametrize('lens,klens', [((1, 63, 64, 65), None), ((127, 128, 129), None), ((300, 1, 515), None), ((1024, ), None), ((5, 130, 1), (260, 130, 129))])
+@pytest.mark.parametrize('causal', [True, False])
+def test_flash_backward_tiles(E, hq, hkv, lens, klens, causal):
+    """Gradients around tile edges (128), for heads that are and are not shared out over a cluster (groups of 1, 3, 4, 8; few and many tiles), keys that
+    are longer than their queries."""
+    from twinkle_b200 import ops
+    g = torch.Generator(device='cuda').manual_seed(hq + sum(lens))
+    klens = klens or lens
+    D, T, Tk = 128, sum(lens), sum(klens)
+    q, k, v, do = (torch.randn(n, h, D, device='cuda', generator=g).bfloat16() for n, h in ((T, hq), (Tk, hkv), (Tk, hkv), (T, hq)))
+    cu, cuk = (torch.tensor([0] + list(x), device='cuda').cumsum(0).int() for x in (lens, klens))
+    leaves = [t.clone().requires_grad_() for t in (q, k, v)]
+    o = ops.flash_attn_varlen(*leaves, cu, max(lens), causal=causal, cu_seqlens_k=cuk, max_seqlen_k=max(klens))
+    got = torch.autograd.grad(o, leaves, do)
+    ref = [t.double().requires_grad_() for t in (q, k, v)]
+    outs, a, b = [], 0, 0
+    for n, m in zip(lens, klens):
+        kk, vv = (t[b:b + m].repeat_interleave(hq // hkv, 1) for t in ref[1:])
+        s = torch.einsum('qhd,khd->hqk', ref[0][a:a + n], kk) * D ** -0.5
+        if causal:
+            s = s.masked_fill(torch.ones(n, m, dtype=torch.bool, device='cuda').triu(m - n + 1), float('-inf'))
+        outs.append(torch.einsum('hqk,khd->qhd', torch.softmax(s, -1), vv))
+        a, b = a + n, b + m
+    want = torch.autograd.grad(torch.cat(outs), ref, do.double())
+    for x, y in zip(got, want):
+        assert rel(x, y) < 8e-3        # P and dS rounded to bf16 (2^-9 each at most) and the result too
+    assert E.read_and_clear_error() == 0

@@ -1,19 +1,29 @@
 // Flash-attention backward for sm_100a (causal, GQA, packed varlen, D = 128), two tcgen05 kernels:
 //
 //   flash_bwd_dkdv_kernel : one CTA per (128-row K/V tile, kv head).  Loops over the query heads of the
-//       GQA group and over 64-row query blocks:  Sᵀ = K·Qᵀ, dPᵀ = V·dOᵀ (tensor cores → TMEM),
-//       Pᵀ = exp2(Sᵀ·c − lse), dSᵀ = Pᵀ∘(dPᵀ − δ) (registers → swizzled smem), dV += Pᵀ·dO, dK += dSᵀ·Q.
+//       GQA group and over 128-row query blocks:  Sᵀ = K·Qᵀ, dPᵀ = V·dOᵀ (tensor cores → TMEM),
+//       Pᵀ = exp2(Sᵀ·c − lse), dSᵀ = Pᵀ∘(dPᵀ − δ) (registers → TMEM), dV += Pᵀ·dO, dK += dSᵀ·Q.
 //       dK/dV of the whole group accumulate in TMEM → no atomics, deterministic.
-//   flash_bwd_dq_kernel   : one CTA per (128-row query tile, query head).  Loops over 64-row K/V blocks:
+//   flash_bwd_dq_kernel   : one CTA per (128-row query tile, query head).  Loops over 128-row K/V blocks:
 //       S = Q·Kᵀ, dP = dO·Vᵀ, dS = P∘(dP − δ), dQ += dS·K.
 //   flash_bwd_delta_kernel: δ[h,t] = Σ_d O·dO.
 // Recomputing S/dP in both kernels costs 7 instead of 5 GEMMs per tile pair but keeps every
 // accumulator on chip without cross-CTA reductions.
+//
+// What bounds them: the tensor cores, by products of 128x128x16 at 64 cycles.  (Blocks of 64 rows had products that take as long for half the
+// work, and two barriers per block on the only path.)  P and dS go back into the TMEM columns of the scores they come from, as the A operand of the
+// accumulating products, which leaves shared memory for two stages of 128-row blocks; each WG writes inside the columns that it alone
+// reads.  Products that do not wait for the arithmetic in progress run under it: dV and the next Sᵀ while dSᵀ is formed, dK and the next
+// dPᵀ while the next Pᵀ is; the next S and dP while dS is.  Products run over K in steps of 16 in the same order as with blocks of 64.
+// 32768 tokens in documents of 0.5-8 k, 32/8 heads, us before → now (TFLOP/s of all products): dK/dV 6320 → 3360 (830), dQ 3990 → 2220 (940);
+// 8 x 4096, 32/4 heads: 5040 → 2590, 3140 → 1730.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <cooperative_groups.h>
 #include <torch/types.h>
 
 #include "common.cuh"
+#include "elect.cuh"
 #include "host.h"
 
 namespace tk {
@@ -22,20 +32,16 @@ using bf16 = __nv_bfloat16;
 CUtensorMap make_head_tmap(const torch::Tensor& t, int rows);
 
 namespace fb {
-constexpr int D = 128, BT = 128 /*outer tile rows*/, BI = 64 /*inner block rows*/;
-constexpr int OUTER_BYTES = BT * D * 2;       // 32 KiB (two [128][64] atoms)
-constexpr int OUTER_ATOM = BT * 64 * 2;       // 16 KiB
-constexpr int INNER_BYTES = BI * D * 2;       // 16 KiB (two [64][64] atoms)
-constexpr int INNER_ATOM = BI * 64 * 2;       // 8 KiB
-constexpr int PT_BYTES = BT * BI * 2;         // 16 KiB ([128][64] atom)
-constexpr int THREADS = 320;  // warps 0-7 compute (two groups of 4, each takes half of the inner-block columns), 8 producer, 9 MMA
-// dkdv: K, V (outer) | Q×2, dO×2 (inner) | Pᵀ, dSᵀ | lse/delta staging | barriers
-constexpr int KV_SMEM_K = 0, KV_SMEM_V = OUTER_BYTES, KV_SMEM_Q = 2 * OUTER_BYTES, KV_SMEM_DO = KV_SMEM_Q + 2 * INNER_BYTES,
-              KV_SMEM_PT = KV_SMEM_DO + 2 * INNER_BYTES, KV_SMEM_DST = KV_SMEM_PT + PT_BYTES, KV_SMEM_STAT = KV_SMEM_DST + PT_BYTES,
-              KV_SMEM_BAR = KV_SMEM_STAT + 2 * 2 * BI * 4, KV_SMEM_TOTAL = KV_SMEM_BAR + 256 + 1024;
-// dq: Q, dO (outer) | K×2, V×2 (inner) | dS | barriers
-constexpr int DQ_SMEM_Q = 0, DQ_SMEM_DO = OUTER_BYTES, DQ_SMEM_K = 2 * OUTER_BYTES, DQ_SMEM_V = DQ_SMEM_K + 2 * INNER_BYTES,
-              DQ_SMEM_DS = DQ_SMEM_V + 2 * INNER_BYTES, DQ_SMEM_BAR = DQ_SMEM_DS + PT_BYTES, DQ_SMEM_TOTAL = DQ_SMEM_BAR + 256 + 1024;
+constexpr int D = 128, BT = 128;              // width, rows of a tile and of a block
+constexpr int TILE_BYTES = BT * D * 2;        // 32 KiB (two [128][64] atoms)
+constexpr int ATOM = BT * 64 * 2;             // 16 KiB
+constexpr int THREADS = 320;  // warps 0-7 compute (two groups of 4, each takes half of a block's columns), 8 producer, 9 MMA
+// two tiles that stay (A, B), two streams of blocks in two stages each (X, Y), lse / δ of a block, barriers.  dK/dV: K, V | Q, dO; dQ: Q, dO | K, V
+constexpr int SMEM_A = 0, SMEM_B = TILE_BYTES, SMEM_X = 2 * TILE_BYTES, SMEM_Y = SMEM_X + 2 * TILE_BYTES, SMEM_STAT = SMEM_Y + 2 * TILE_BYTES,
+              SMEM_BAR = SMEM_STAT + 2 * 2 * BT * 4, SMEM_TOTAL = SMEM_BAR + 256 + 1024;
+constexpr int SUM_PITCH = D + 4;              // floats between rows of a partial sum
+static_assert(2 * BT * SUM_PITCH * 4 <= SMEM_STAT, "partial sums lie over the tiles");
+__device__ __forceinline__ constexpr uint32_t step(int k) { return ((k >> 2) * ATOM + (k & 3) * 32) >> 4; }   // of a K-major operand, 16 along K, in a descriptor
 }  // namespace fb
 
 struct BwdParams {
@@ -68,35 +74,40 @@ __global__ void flash_bwd_delta_kernel(const bf16* __restrict__ o, const bf16* _
 }
 
 // ============================================================== dK / dV
+// SPLIT: a cluster of gridDim.x / hkv CTAs shares a tile by query heads and adds up through distributed shared memory.
+template <bool SPLIT>
 __global__ void __launch_bounds__(fb::THREADS, 1)
 flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmDO, const BwdParams p) {
   using namespace fb;
-  const int kv_head = blockIdx.x, seq = blockIdx.z;
+  namespace cg = cooperative_groups;
+  const int parts = SPLIT ? gridDim.x / p.hkv : 1;
+  const int kv_head = blockIdx.x / parts, rank = blockIdx.x % parts, seq = blockIdx.z;
   const int seq_start = p.cu[seq], seq_len = p.cu[seq + 1] - seq_start;          // queries
   const int kv_start = p.cu_k[seq], kv_len = p.cu_k[seq + 1] - kv_start;         // keys / values
   const int q_off = kv_len - seq_len;            // causal: query row r sees keys 0 … r + q_off
   const int n_tiles = (kv_len + BT - 1) / BT;
   if (static_cast<int>(blockIdx.y) >= n_tiles) return;
   const int kv0 = blockIdx.y * BT;               // early tiles have the most query blocks → scheduled first
-  const int G = p.hq / p.hkv;
-  const int qb_end = (seq_len + BI - 1) / BI;
-  const int qb_begin = p.causal ? min(max(kv0 - q_off, 0) / BI, qb_end) : 0;
+  const int G = p.hq / p.hkv, heads = G / parts, head0 = kv_head * G + rank * heads;
+  const int qb_end = (seq_len + BT - 1) / BT;
+  const int qb_begin = p.causal ? min(max(kv0 - q_off, 0) / BT, qb_end) : 0;
   const int per_head = qb_end - qb_begin;
-  const int n_iter = per_head * G;
+  const int n_iter = per_head * heads;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + KV_SMEM_BAR);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SMEM_BAR);
   uint64_t* kv_full = bars;          // 1
   uint64_t* qdo_full = bars + 1;     // 2
   uint64_t* qdo_empty = bars + 3;    // 2
-  uint64_t* sd_full = bars + 5;      // 2
-  uint64_t* sd_empty = bars + 7;     // 2
-  uint64_t* pds_ready = bars + 9;    // 1
-  uint64_t* acc_done = bars + 10;    // 1
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
-  float* stat = reinterpret_cast<float*>(smem + KV_SMEM_STAT);  // [2 buffers][lse2 | delta][64]
+  uint64_t* s_full = bars + 5;
+  uint64_t* dp_full = bars + 6;
+  uint64_t* p_ready = bars + 7;
+  uint64_t* ds_ready = bars + 8;
+  uint64_t* acc_done = bars + 9;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
+  float* stat = reinterpret_cast<float*>(smem + SMEM_STAT);  // [2 buffers][lse2 | delta][128]
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -104,10 +115,11 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     for (int i = 0; i < 2; ++i) {
       mbar_init(&qdo_full[i], 1);
       mbar_init(&qdo_empty[i], 1);
-      mbar_init(&sd_full[i], 1);
-      mbar_init(&sd_empty[i], 256);
     }
-    mbar_init(pds_ready, 256);
+    mbar_init(s_full, 1);
+    mbar_init(dp_full, 1);
+    mbar_init(p_ready, 256);
+    mbar_init(ds_ready, 256);
     mbar_init(acc_done, 1);
     fence_barrier_init();
   }
@@ -119,17 +131,17 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
-  // TMEM columns: Sᵀ buffers [0,64) [64,128); dPᵀ buffers [128,192) [192,256); dV [256,384); dK [384,512)
-  const uint32_t t_dv = tmem_base + 256, t_dk = tmem_base + 384;
+  // TMEM columns: Sᵀ [0,128), of which Pᵀ takes [0,32) and [64,96); dPᵀ [128,256), dSᵀ inside it likewise; dV [256,384); dK [384,512)
+  const uint32_t t_s = tmem_base, t_dp = tmem_base + 128, t_dv = tmem_base + 256, t_dk = tmem_base + 384;
 
   if (warp == 8) {
     // producer warp: lane 0 drives TMA; all lanes stage lse (log2 units) and δ of each query block in smem
     if (lane == 0) {
-      mbar_expect_tx(kv_full, 2 * OUTER_BYTES);
-      tma_load_3d(smem + KV_SMEM_K, &tmK, kv_full, 0, kv_head, kv_start + kv0);
-      tma_load_3d(smem + KV_SMEM_K + OUTER_ATOM, &tmK, kv_full, 64, kv_head, kv_start + kv0);
-      tma_load_3d(smem + KV_SMEM_V, &tmV, kv_full, 0, kv_head, kv_start + kv0);
-      tma_load_3d(smem + KV_SMEM_V + OUTER_ATOM, &tmV, kv_full, 64, kv_head, kv_start + kv0);
+      mbar_expect_tx(kv_full, 2 * TILE_BYTES);
+      tma_load_3d(smem + SMEM_A, &tmK, kv_full, 0, kv_head, kv_start + kv0);
+      tma_load_3d(smem + SMEM_A + ATOM, &tmK, kv_full, 64, kv_head, kv_start + kv0);
+      tma_load_3d(smem + SMEM_B, &tmV, kv_full, 0, kv_head, kv_start + kv0);
+      tma_load_3d(smem + SMEM_B + ATOM, &tmV, kv_full, 64, kv_head, kv_start + kv0);
     }
     for (int it = 0; it < n_iter; ++it) {
       const int st = it & 1;
@@ -139,9 +151,10 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         ok = __shfl_sync(0xffffffffu, ok, 0);
         if (!ok) break;
       }
-      const int head = kv_head * G + it / per_head;
-      const int qb0 = (qb_begin + it % per_head) * BI;
-      for (int c = lane; c < BI; c += 32) {
+      const int head = head0 + it / per_head;
+      const int qb0 = (qb_begin + it % per_head) * BT;
+#pragma unroll
+      for (int c = lane; c < BT; c += 32) {
         const int qpos = qb0 + c;
         float l2 = INFINITY, dl = 0.f;   // exp2(s − inf) = 0 for query rows past the end of the sequence
         if (qpos < seq_len) {
@@ -149,137 +162,166 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           l2 = p.lse[idx] * 1.4426950408889634f;
           dl = p.delta[idx];
         }
-        stat[st * 2 * BI + c] = l2;
-        stat[st * 2 * BI + BI + c] = dl;
+        stat[st * 2 * BT + c] = -l2;
+        stat[st * 2 * BT + BT + c] = -dl;
       }
       __syncwarp();
       if (lane == 0) {
         const int row = seq_start + qb0;
-        mbar_expect_tx(&qdo_full[st], 2 * INNER_BYTES);
-        tma_load_3d(smem + KV_SMEM_Q + st * INNER_BYTES, &tmQ, &qdo_full[st], 0, head, row);
-        tma_load_3d(smem + KV_SMEM_Q + st * INNER_BYTES + INNER_ATOM, &tmQ, &qdo_full[st], 64, head, row);
-        tma_load_3d(smem + KV_SMEM_DO + st * INNER_BYTES, &tmDO, &qdo_full[st], 0, head, row);
-        tma_load_3d(smem + KV_SMEM_DO + st * INNER_BYTES + INNER_ATOM, &tmDO, &qdo_full[st], 64, head, row);
+        mbar_expect_tx(&qdo_full[st], 2 * TILE_BYTES);
+        tma_load_3d(smem + SMEM_X + st * TILE_BYTES, &tmQ, &qdo_full[st], 0, head, row);
+        tma_load_3d(smem + SMEM_X + st * TILE_BYTES + ATOM, &tmQ, &qdo_full[st], 64, head, row);
+        tma_load_3d(smem + SMEM_Y + st * TILE_BYTES, &tmDO, &qdo_full[st], 0, head, row);
+        tma_load_3d(smem + SMEM_Y + st * TILE_BYTES + ATOM, &tmDO, &qdo_full[st], 64, head, row);
       }
     }
   } else if (warp == 9) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = umma_idesc_bf16(BT, BI, false, false);   // [128 kv] x [64 q], K = d
-      constexpr uint32_t idesc_acc = umma_idesc_bf16(BT, D, false, true);   // [128 kv] x [128 d], K = q (B MN-major)
-      const uint32_t sk = smem_u32(smem + KV_SMEM_K), sv = smem_u32(smem + KV_SMEM_V);
-      const uint32_t spt = smem_u32(smem + KV_SMEM_PT), sdst = smem_u32(smem + KV_SMEM_DST);
-      auto issue_sd = [&](int it) {
-        const int st = it & 1;
-        const uint32_t sq = smem_u32(smem + KV_SMEM_Q + st * INNER_BYTES), sdo = smem_u32(smem + KV_SMEM_DO + st * INNER_BYTES);
+    // the whole warp walks the loop and one thread issues: descriptors stay in uniform registers
+    constexpr uint32_t idesc_s = umma_idesc_bf16(BT, BT, false, false);   // [128 kv] x [128 q], K = d
+    constexpr uint32_t idesc_acc = umma_idesc_bf16(BT, D, false, true);   // [128 kv] x [128 d], K = q (B MN-major)
+    const uint64_t dK = umma_desc(smem_u32(smem + SMEM_A), 16, 1024), dV = umma_desc(smem_u32(smem + SMEM_B), 16, 1024);
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.err, ERR_ATTN_WAIT)); };
+    auto scores = [&](uint32_t d, uint64_t a, int at, uint64_t* bar) {       // d = a · (tile at `at`)ᵀ
+      const uint64_t b = umma_desc(smem_u32(smem + at), 16, 1024);
+      if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t offA = (k >> 2) * OUTER_ATOM + (k & 3) * 32, offB = (k >> 2) * INNER_ATOM + (k & 3) * 32;
-          umma_bf16(tmem_base + st * 64, umma_desc(sk + offA, 16, 1024), umma_desc(sq + offB, 16, 1024), idesc_s, k ? 1u : 0u);
-        }
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t offA = (k >> 2) * OUTER_ATOM + (k & 3) * 32, offB = (k >> 2) * INNER_ATOM + (k & 3) * 32;
-          umma_bf16(tmem_base + 128 + st * 64, umma_desc(sv + offA, 16, 1024), umma_desc(sdo + offB, 16, 1024), idesc_s, k ? 1u : 0u);
-        }
-        umma_commit(&sd_full[st]);
-      };
-      bool ok = n_iter > 0 && mbar_wait(kv_full, 0, p.err, ERR_ATTN_WAIT) && mbar_wait(&qdo_full[0], 0, p.err, ERR_ATTN_WAIT);
-      if (ok) {
-        tc_fence_after();
-        issue_sd(0);
+        for (int k = 0; k < D / 16; ++k) umma_bf16(d, a + step(k), b + step(k), idesc_s, k ? 1u : 0u);
+        umma_commit(bar);
       }
-      for (int it = 0; ok && it < n_iter; ++it) {
-        if (it + 1 < n_iter) {
-          const int n = it + 1;
-          ok = mbar_wait(&qdo_full[n & 1], (n >> 1) & 1, p.err, ERR_ATTN_WAIT);
-          if (ok && n >= 2) ok = mbar_wait(&sd_empty[n & 1], ((n >> 1) - 1) & 1, p.err, ERR_ATTN_WAIT);
-          if (!ok) break;
-          tc_fence_after();
-          issue_sd(n);
-        }
-        if (!mbar_wait(pds_ready, it & 1, p.err, ERR_ATTN_WAIT)) break;
-        tc_fence_after();
-        const int st = it & 1;
-        const uint32_t sq = smem_u32(smem + KV_SMEM_Q + st * INNER_BYTES), sdo = smem_u32(smem + KV_SMEM_DO + st * INNER_BYTES);
+      __syncwarp();
+    };
+    auto add_up = [&](uint32_t d, uint32_t a, int at, bool first, uint64_t* bar) {      // d += a (tensor memory) · tile
+      const uint64_t b = umma_desc(smem_u32(smem + at), ATOM, 1024);
+      if (elect_one()) {
+        const uint32_t add = !first;
 #pragma unroll
-        for (int k = 0; k < BI / 16; ++k)   // dV += Pᵀ·dO
-          umma_bf16(t_dv, umma_desc(spt + k * 32, 16, 1024), umma_desc(sdo + k * 2048, INNER_ATOM, 1024), idesc_acc, (it > 0 || k > 0) ? 1u : 0u);
-#pragma unroll
-        for (int k = 0; k < BI / 16; ++k)   // dK += dSᵀ·Q
-          umma_bf16(t_dk, umma_desc(sdst + k * 32, 16, 1024), umma_desc(sq + k * 2048, INNER_ATOM, 1024), idesc_acc, (it > 0 || k > 0) ? 1u : 0u);
-        umma_commit(acc_done);
-        umma_commit(&qdo_empty[st]);
+        for (int k = 0; k < BT / 16; ++k) umma_bf16_ts(d, a + (k >> 2) * 64 + (k & 3) * 8, b + k * 128, idesc_acc, k > 0 ? 1u : add);
+        if (bar != nullptr) umma_commit(bar);
       }
-    }
-  } else {
-    const int wg = warp >> 2;                       // which half of the 64 inner-block columns this thread handles
-    const int row = (warp & 3) * 32 + lane;
-    const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const int kv_pos = kv0 + row;
-    const bool row_valid = kv_pos < kv_len;
-    bool ok = true;
-    for (int it = 0; it < n_iter; ++it) {
-      const int st = it & 1;
-      const int qb0 = (qb_begin + it % per_head) * BI;
-      if (!mbar_wait(&sd_full[st], (it >> 1) & 1, p.err, ERR_ATTN_WAIT)) { ok = false; break; }
+      __syncwarp();
+    };
+    bool ok = n_iter > 0 && wait(kv_full, 0) && wait(&qdo_full[0], 0);
+    if (ok) {
       tc_fence_after();
-      const float* lse2 = stat + st * 2 * BI;
-      const float* dl = lse2 + BI;
-      {
-        const int c = wg;
-        uint32_t s[32], dp[32];
-        tmem_ld32(tmem_base + st * 64 + c * 32 + lane_off, s);
-        tmem_ld32(tmem_base + 128 + st * 64 + c * 32 + lane_off, dp);
+      scores(t_s, dK, SMEM_X, s_full);
+      scores(t_dp, dV, SMEM_Y, dp_full);
+    }
+    for (int it = 0; ok && it < n_iter; ++it) {
+      const int st = it & 1, nx = st ^ 1;
+      const bool more = it + 1 < n_iter;
+      if (!wait(p_ready, it & 1)) break;
+      tc_fence_after();
+      add_up(t_dv, t_s, SMEM_Y + st * TILE_BYTES, it == 0, nullptr);            // dV += Pᵀ·dO
+      if (more) {
+        if (!wait(&qdo_full[nx], ((it + 1) >> 1) & 1)) break;
+        tc_fence_after();
+        scores(t_s, dK, SMEM_X + nx * TILE_BYTES, s_full);                       // runs after the product that reads Pᵀ
+      }
+      if (!wait(ds_ready, it & 1)) break;
+      tc_fence_after();
+      add_up(t_dk, t_dp, SMEM_X + st * TILE_BYTES, it == 0, &qdo_empty[st]);    // dK += dSᵀ·Q
+      if (more) scores(t_dp, dV, SMEM_Y + nx * TILE_BYTES, dp_full);
+    }
+    if (elect_one()) umma_commit(acc_done);
+    __syncwarp();
+  }
+  bool ok = true;
+  const int wg = warp >> 2;                       // which half of the 128 queries of a block this thread handles
+  const int row = (warp & 3) * 32 + lane;
+  const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
+  const int kv_pos = kv0 + row;
+  const bool row_valid = kv_pos < kv_len;
+  if (warp < 8) {
+    const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
+    for (int it = 0; it < n_iter; ++it) {
+      const int qb0 = (qb_begin + it % per_head) * BT + wg * 64;
+      const float* lse2 = stat + (it & 1) * 2 * BT + wg * 64;       // negated, as is δ
+      const float* dl = lse2 + BT;
+      if (!mbar_wait(s_full, it & 1, p.err, ERR_ATTN_WAIT)) { ok = false; break; }
+      tc_fence_after();
+      // only blocks that touch the causal diagonal need per-element masking; rows past the end of the keys are
+      // zeroed wholesale; query rows past the end carry lse = +inf and vanish through exp2
+      const bool diag = p.causal && (qb0 + q_off < kv0 + BT - 1);
+      float pr[64];
+      uint32_t pk[32];
+#pragma unroll
+      for (int c = 0; c < 64; c += 32) {
+        uint32_t s[32];
+        tmem_ld32(t_s + wg * 64 + c + lane_off, s);
         tmem_ld_wait();
-        uint32_t pk[16], dsk[16];
-        // only blocks that touch the causal diagonal need per-element masking; rows past the end of the keys are
-        // zeroed wholesale; query rows past the end carry lse = +inf and vanish through exp2
-        const bool diag = p.causal && (qb0 + q_off < kv0 + BT - 1);
-        const float4* l4 = reinterpret_cast<const float4*>(lse2 + c * 32);
-        const float4* d4 = reinterpret_cast<const float4*>(dl + c * 32);
+        const float4* l4 = reinterpret_cast<const float4*>(lse2 + c);
 #pragma unroll
         for (int i = 0; i < 32; i += 4) {
-          const float4 lv = l4[i >> 2], dv4 = d4[i >> 2];
-          const float ls[4] = {lv.x, lv.y, lv.z, lv.w}, ds[4] = {dv4.x, dv4.y, dv4.z, dv4.w};
-          float pv[4], dv[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            float pr = fast_exp2(__uint_as_float(s[i + e]) * p.scale_log2 - ls[e]);
-            if (diag && (qb0 + c * 32 + i + e + q_off < kv_pos)) pr = 0.f;
-            pv[e] = pr;
-            dv[e] = pr * (__uint_as_float(dp[i + e]) - ds[e]);
-          }
-          pk[i >> 1] = pack_bf16(pv[0], pv[1]);
-          pk[(i >> 1) + 1] = pack_bf16(pv[2], pv[3]);
-          dsk[i >> 1] = pack_bf16(dv[0], dv[1]);
-          dsk[(i >> 1) + 1] = pack_bf16(dv[2], dv[3]);
+          const float4 l = l4[i >> 2];
+          const float2 x = fma2(make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), scale2, make_float2(l.x, l.y));
+          const float2 y = fma2(make_float2(__uint_as_float(s[i + 2]), __uint_as_float(s[i + 3])), scale2, make_float2(l.z, l.w));
+          pr[c + i] = fast_exp2(x.x);
+          pr[c + i + 1] = fast_exp2(x.y);
+          pr[c + i + 2] = fast_exp2(y.x);
+          pr[c + i + 3] = fast_exp2(y.y);
         }
-        if (!row_valid) {
-#pragma unroll
-          for (int i = 0; i < 16; ++i) { pk[i] = 0u; dsk[i] = 0u; }
-        }
-        // S/dP are in registers: the TMEM buffers can be refilled while we finish
-        tc_fence_before();
-        mbar_arrive(&sd_empty[st]);
-        // Pᵀ / dSᵀ smem is free once the accumulating MMAs of the previous iteration retired
-        if (it > 0 && !mbar_wait(acc_done, (it - 1) & 1, p.err, ERR_ATTN_WAIT)) { ok = false; break; }
-        store_row_chunk_sw128(smem + KV_SMEM_PT, 128, row, c * 32, pk);
-        store_row_chunk_sw128(smem + KV_SMEM_DST, 128, row, c * 32, dsk);
       }
-      fence_proxy_async();
-      mbar_arrive(pds_ready);
-    }
-    if (ok && n_iter > 0 && mbar_wait(acc_done, (n_iter - 1) & 1, p.err, ERR_ATTN_WAIT)) {
+      if (diag) {
+        const int gone = kv_pos - q_off - qb0;      // queries before this one of the half do not see the key
+#pragma unroll
+        for (int i = 0; i < 64; ++i)
+          if (i < gone) pr[i] = 0.f;
+      }
+      if (!row_valid) {
+#pragma unroll
+        for (int i = 0; i < 64; ++i) pr[i] = 0.f;
+      }
+#pragma unroll
+      for (int i = 0; i < 32; ++i) pk[i] = pack_bf16(pr[2 * i], pr[2 * i + 1]);
+      tmem_st32(t_s + wg * 64 + lane_off, pk);
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(p_ready);
+      if (!mbar_wait(dp_full, it & 1, p.err, ERR_ATTN_WAIT)) { ok = false; break; }
       tc_fence_after();
-      bf16* dkrow = p.dk + (static_cast<size_t>(kv_start + kv_pos) * p.hkv + kv_head) * D;
-      bf16* dvrow = p.dv + (static_cast<size_t>(kv_start + kv_pos) * p.hkv + kv_head) * D;
+#pragma unroll
+      for (int c = 0; c < 64; c += 32) {
+        uint32_t dp[32];
+        tmem_ld32(t_dp + wg * 64 + c + lane_off, dp);
+        tmem_ld_wait();
+        const float4* d4 = reinterpret_cast<const float4*>(dl + c);
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+          const float4 d = d4[i >> 2];
+          const float2 x = mul2(make_float2(pr[c + i], pr[c + i + 1]), add2(make_float2(__uint_as_float(dp[i]), __uint_as_float(dp[i + 1])), make_float2(d.x, d.y)));
+          const float2 y = mul2(make_float2(pr[c + i + 2], pr[c + i + 3]), add2(make_float2(__uint_as_float(dp[i + 2]), __uint_as_float(dp[i + 3])), make_float2(d.z, d.w)));
+          pk[(c + i) >> 1] = pack_bf16(x.x, x.y);
+          pk[((c + i) >> 1) + 1] = pack_bf16(y.x, y.y);
+        }
+      }
+      if (!row_valid) {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) pk[i] = 0u;
+      }
+      tmem_st32(t_dp + wg * 64 + lane_off, pk);
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(ds_ready);
+    }
+    if (n_iter > 0) ok = ok && mbar_wait(acc_done, 0, p.err, ERR_ATTN_WAIT);
+    tc_fence_after();
+    bf16* dkrow = p.dk + (static_cast<size_t>(kv_start + kv_pos) * p.hkv + kv_head) * D;
+    bf16* dvrow = p.dv + (static_cast<size_t>(kv_start + kv_pos) * p.hkv + kv_head) * D;
+    if (ok && n_iter > 0) {
 #pragma unroll 1
       for (int c = 2 * wg; c < 2 * wg + 2; ++c) {
         uint32_t a[32], b[32];
         tmem_ld32(t_dv + lane_off + c * 32, a);
         tmem_ld32(t_dk + lane_off + c * 32, b);
         tmem_ld_wait();
-        if (row_valid) {
+        if constexpr (SPLIT) {        // the tiles are read for the last time: their place takes the sums, dV then dK
+          float* mine = reinterpret_cast<float*>(smem) + row * SUM_PITCH + c * 32;
+#pragma unroll
+          for (int i = 0; i < 32; i += 4) {
+            *reinterpret_cast<uint4*>(mine + i) = make_uint4(a[i], a[i + 1], a[i + 2], a[i + 3]);
+            *reinterpret_cast<uint4*>(mine + BT * SUM_PITCH + i) = make_uint4(b[i], b[i + 1], b[i + 2], b[i + 3]);
+          }
+        } else if (row_valid) {
 #pragma unroll
           for (int i = 0; i < 32; i += 8) {
             *reinterpret_cast<uint4*>(dvrow + c * 32 + i) =
@@ -293,15 +335,32 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
           }
         }
       }
-    } else if (n_iter == 0 && row_valid) {
+    } else if (n_iter == 0 && row_valid && rank == 0) {
       // no query attends to this tile (cannot happen with causal self-attention, kept for safety)
-      bf16* dkrow = p.dk + (static_cast<size_t>(kv_start + kv_pos) * p.hkv + kv_head) * D;
-      bf16* dvrow = p.dv + (static_cast<size_t>(kv_start + kv_pos) * p.hkv + kv_head) * D;
       for (int i = wg * 64; i < wg * 64 + 64; i += 8) {
         *reinterpret_cast<uint4*>(dkrow + i) = make_uint4(0, 0, 0, 0);
         *reinterpret_cast<uint4*>(dvrow + i) = make_uint4(0, 0, 0, 0);
       }
     }
+  }
+  if constexpr (SPLIT) {
+    const cg::cluster_group cluster = cg::this_cluster();
+    cluster.sync();
+    if (n_iter > 0) {
+      const float* sums = reinterpret_cast<const float*>(smem);
+      for (int i = rank * THREADS + threadIdx.x; i < 2 * BT * (D / 4); i += parts * THREADS) {
+        const int which = i / (BT * (D / 4)), r = i / (D / 4) % BT, c = i % (D / 4) * 4;
+        if (kv0 + r >= kv_len) continue;
+        float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int k = 0; k < parts; ++k) {
+          const float4 v = *reinterpret_cast<const float4*>(cluster.map_shared_rank(sums, k) + (which * BT + r) * SUM_PITCH + c);
+          s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+        }
+        const float f = which ? p.scale : 1.f;
+        *reinterpret_cast<uint2*>((which ? p.dk : p.dv) + (static_cast<size_t>(kv_start + kv0 + r) * p.hkv + kv_head) * D + c) = make_uint2(pack_bf16(s.x * f, s.y * f), pack_bf16(s.z * f, s.w * f));
+      }
+    }
+    cluster.sync();
   }
   tc_fence_before();
   __syncthreads();
@@ -325,19 +384,19 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int kv_start = p.cu_k[seq], kv_len = p.cu_k[seq + 1] - kv_start;
   const int q_off = kv_len - seq_len;
   const int kv_end = p.causal ? max(0, min(kv_len, q0 + BT + q_off)) : kv_len;
-  const int n_iter = (kv_end + BI - 1) / BI;
+  const int n_iter = (kv_end + BT - 1) / BT;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + DQ_SMEM_BAR);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SMEM_BAR);
   uint64_t* qdo_full = bars;         // 1
   uint64_t* kv_full = bars + 1;      // 2
   uint64_t* kv_empty = bars + 3;     // 2
-  uint64_t* sd_full = bars + 5;      // 2
-  uint64_t* sd_empty = bars + 7;     // 2
-  uint64_t* ds_ready = bars + 9;     // 1
-  uint64_t* acc_done = bars + 10;    // 1
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 11);
+  uint64_t* sd_full = bars + 5;
+  uint64_t* dp_empty = bars + 6;
+  uint64_t* ds_ready = bars + 7;     // 2
+  uint64_t* acc_done = bars + 9;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 10);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -345,10 +404,10 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     for (int i = 0; i < 2; ++i) {
       mbar_init(&kv_full[i], 1);
       mbar_init(&kv_empty[i], 1);
-      mbar_init(&sd_full[i], 1);
-      mbar_init(&sd_empty[i], 256);
+      mbar_init(&ds_ready[i], 256);
     }
-    mbar_init(ds_ready, 256);
+    mbar_init(sd_full, 1);
+    mbar_init(dp_empty, 256);
     mbar_init(acc_done, 1);
     fence_barrier_init();
   }
@@ -360,71 +419,71 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
-  // TMEM columns: S buffers [0,64) [64,128); dP buffers [128,192) [192,256); dQ [256,384)
-  const uint32_t t_dq = tmem_base + 256;
+  // TMEM columns: S in two buffers [0,128) [128,256), of which dS takes [0,32) and [64,96); dP [256,384); dQ [384,512)
+  const uint32_t t_dp = tmem_base + 256, t_dq = tmem_base + 384;
 
   if (warp == 8) {
     if (lane == 0) {
-      mbar_expect_tx(qdo_full, 2 * OUTER_BYTES);
-      tma_load_3d(smem + DQ_SMEM_Q, &tmQ, qdo_full, 0, head, seq_start + q0);
-      tma_load_3d(smem + DQ_SMEM_Q + OUTER_ATOM, &tmQ, qdo_full, 64, head, seq_start + q0);
-      tma_load_3d(smem + DQ_SMEM_DO, &tmDO, qdo_full, 0, head, seq_start + q0);
-      tma_load_3d(smem + DQ_SMEM_DO + OUTER_ATOM, &tmDO, qdo_full, 64, head, seq_start + q0);
+      mbar_expect_tx(qdo_full, 2 * TILE_BYTES);
+      tma_load_3d(smem + SMEM_A, &tmQ, qdo_full, 0, head, seq_start + q0);
+      tma_load_3d(smem + SMEM_A + ATOM, &tmQ, qdo_full, 64, head, seq_start + q0);
+      tma_load_3d(smem + SMEM_B, &tmDO, qdo_full, 0, head, seq_start + q0);
+      tma_load_3d(smem + SMEM_B + ATOM, &tmDO, qdo_full, 64, head, seq_start + q0);
       for (int it = 0; it < n_iter; ++it) {
         const int st = it & 1;
         if (it >= 2 && !mbar_wait(&kv_empty[st], ((it >> 1) - 1) & 1, p.err, ERR_ATTN_WAIT)) break;
-        const int row = kv_start + it * BI;
-        mbar_expect_tx(&kv_full[st], 2 * INNER_BYTES);
-        tma_load_3d(smem + DQ_SMEM_K + st * INNER_BYTES, &tmK, &kv_full[st], 0, kv_head, row);
-        tma_load_3d(smem + DQ_SMEM_K + st * INNER_BYTES + INNER_ATOM, &tmK, &kv_full[st], 64, kv_head, row);
-        tma_load_3d(smem + DQ_SMEM_V + st * INNER_BYTES, &tmV, &kv_full[st], 0, kv_head, row);
-        tma_load_3d(smem + DQ_SMEM_V + st * INNER_BYTES + INNER_ATOM, &tmV, &kv_full[st], 64, kv_head, row);
+        const int row = kv_start + it * BT;
+        mbar_expect_tx(&kv_full[st], 2 * TILE_BYTES);
+        tma_load_3d(smem + SMEM_X + st * TILE_BYTES, &tmK, &kv_full[st], 0, kv_head, row);
+        tma_load_3d(smem + SMEM_X + st * TILE_BYTES + ATOM, &tmK, &kv_full[st], 64, kv_head, row);
+        tma_load_3d(smem + SMEM_Y + st * TILE_BYTES, &tmV, &kv_full[st], 0, kv_head, row);
+        tma_load_3d(smem + SMEM_Y + st * TILE_BYTES + ATOM, &tmV, &kv_full[st], 64, kv_head, row);
       }
     }
   } else if (warp == 9) {
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = umma_idesc_bf16(BT, BI, false, false);   // [128 q] x [64 kv], K = d
-      constexpr uint32_t idesc_acc = umma_idesc_bf16(BT, D, false, true);   // [128 q] x [128 d], K = kv (B MN-major)
-      const uint32_t sq = smem_u32(smem + DQ_SMEM_Q), sdo = smem_u32(smem + DQ_SMEM_DO), sds = smem_u32(smem + DQ_SMEM_DS);
-      auto issue_sd = [&](int it) {
-        const int st = it & 1;
-        const uint32_t sk = smem_u32(smem + DQ_SMEM_K + st * INNER_BYTES), sv = smem_u32(smem + DQ_SMEM_V + st * INNER_BYTES);
+    constexpr uint32_t idesc_s = umma_idesc_bf16(BT, BT, false, false);   // [128 q] x [128 kv], K = d
+    constexpr uint32_t idesc_acc = umma_idesc_bf16(BT, D, false, true);   // [128 q] x [128 d], K = kv (B MN-major)
+    const uint64_t dQ = umma_desc(smem_u32(smem + SMEM_A), 16, 1024), dO = umma_desc(smem_u32(smem + SMEM_B), 16, 1024);
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.err, ERR_ATTN_WAIT)); };
+    auto scores = [&](uint32_t d, uint64_t a, int at, uint64_t* bar) {
+      const uint64_t b = umma_desc(smem_u32(smem + at), 16, 1024);
+      if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t offA = (k >> 2) * OUTER_ATOM + (k & 3) * 32, offB = (k >> 2) * INNER_ATOM + (k & 3) * 32;
-          umma_bf16(tmem_base + st * 64, umma_desc(sq + offA, 16, 1024), umma_desc(sk + offB, 16, 1024), idesc_s, k ? 1u : 0u);
-        }
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t offA = (k >> 2) * OUTER_ATOM + (k & 3) * 32, offB = (k >> 2) * INNER_ATOM + (k & 3) * 32;
-          umma_bf16(tmem_base + 128 + st * 64, umma_desc(sdo + offA, 16, 1024), umma_desc(sv + offB, 16, 1024), idesc_s, k ? 1u : 0u);
-        }
-        umma_commit(&sd_full[st]);
-      };
-      bool ok = n_iter > 0 && mbar_wait(qdo_full, 0, p.err, ERR_ATTN_WAIT) && mbar_wait(&kv_full[0], 0, p.err, ERR_ATTN_WAIT);
-      if (ok) {
-        tc_fence_after();
-        issue_sd(0);
+        for (int k = 0; k < D / 16; ++k) umma_bf16(d, a + step(k), b + step(k), idesc_s, k ? 1u : 0u);
+        if (bar != nullptr) umma_commit(bar);
       }
-      for (int it = 0; ok && it < n_iter; ++it) {
-        if (it + 1 < n_iter) {
-          const int n = it + 1;
-          ok = mbar_wait(&kv_full[n & 1], (n >> 1) & 1, p.err, ERR_ATTN_WAIT);
-          if (ok && n >= 2) ok = mbar_wait(&sd_empty[n & 1], ((n >> 1) - 1) & 1, p.err, ERR_ATTN_WAIT);
-          if (!ok) break;
-          tc_fence_after();
-          issue_sd(n);
-        }
-        if (!mbar_wait(ds_ready, it & 1, p.err, ERR_ATTN_WAIT)) break;
+      __syncwarp();
+    };
+    bool ok = n_iter > 0 && wait(qdo_full, 0) && wait(&kv_full[0], 0);
+    if (ok) {
+      tc_fence_after();
+      scores(tmem_base, dQ, SMEM_X, nullptr);
+      scores(t_dp, dO, SMEM_Y, sd_full);
+    }
+    for (int it = 0; ok && it < n_iter; ++it) {
+      if (it + 1 < n_iter) {
+        const int nx = (it + 1) & 1;
+        if (!wait(&kv_full[nx], ((it + 1) >> 1) & 1)) break;
         tc_fence_after();
-        const uint32_t sk = smem_u32(smem + DQ_SMEM_K + (it & 1) * INNER_BYTES);
+        scores(tmem_base + nx * 128, dQ, SMEM_X + nx * TILE_BYTES, nullptr);     // its buffer's dS was read by the product before
+        if (!wait(dp_empty, it & 1)) break;
+        tc_fence_after();
+        scores(t_dp, dO, SMEM_Y + nx * TILE_BYTES, sd_full);
+      }
+      if (!wait(&ds_ready[it & 1], (it >> 1) & 1)) break;
+      tc_fence_after();
+      const uint64_t k_ = umma_desc(smem_u32(smem + SMEM_X + (it & 1) * TILE_BYTES), ATOM, 1024);
+      if (elect_one()) {
+        const uint32_t add = it > 0;
 #pragma unroll
-        for (int k = 0; k < BI / 16; ++k)   // dQ += dS·K
-          umma_bf16(t_dq, umma_desc(sds + k * 32, 16, 1024), umma_desc(sk + k * 2048, INNER_ATOM, 1024), idesc_acc, (it > 0 || k > 0) ? 1u : 0u);
-        umma_commit(acc_done);
+        for (int k = 0; k < BT / 16; ++k)   // dQ += dS·K
+          umma_bf16_ts(t_dq, tmem_base + (it & 1) * 128 + (k >> 2) * 64 + (k & 3) * 8, k_ + k * 128, idesc_acc, k > 0 ? 1u : add);
         umma_commit(&kv_empty[it & 1]);
       }
+      __syncwarp();
     }
+    if (elect_one()) umma_commit(acc_done);
+    __syncwarp();
   } else {
     const int wg = warp >> 2;
     const int row = (warp & 3) * 32 + lane;
@@ -437,44 +496,45 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       lse2 = p.lse[idx] * 1.4426950408889634f;
       dl = p.delta[idx];
     }
+    const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), lse_2 = make_float2(-lse2, -lse2), dl_2 = make_float2(-dl, -dl);
     bool ok = true;
     for (int it = 0; it < n_iter; ++it) {
-      const int st = it & 1;
-      if (!mbar_wait(&sd_full[st], (it >> 1) & 1, p.err, ERR_ATTN_WAIT)) { ok = false; break; }
+      if (!mbar_wait(sd_full, it & 1, p.err, ERR_ATTN_WAIT)) { ok = false; break; }
       tc_fence_after();
-      const int kvb = it * BI;
-      {
-        const int c = wg;
-        uint32_t s[32], dp[32];
-        tmem_ld32(tmem_base + st * 64 + c * 32 + lane_off, s);
-        tmem_ld32(tmem_base + 128 + st * 64 + c * 32 + lane_off, dp);
+      const int kvb = it * BT + wg * 64;
+      const uint32_t t_s = tmem_base + (it & 1) * 128 + wg * 64 + lane_off;
+      uint32_t dp[64], pk[32];
+      tmem_ld32(t_dp + wg * 64 + lane_off, *reinterpret_cast<uint32_t(*)[32]>(dp));
+      tmem_ld32(t_dp + wg * 64 + 32 + lane_off, *reinterpret_cast<uint32_t(*)[32]>(dp + 32));
+      tmem_ld_wait();
+      tc_fence_before();
+      mbar_arrive(dp_empty);             // the next dP may be formed
+      // masking is needed only where the block crosses the causal diagonal of this query tile or the end of the keys
+      const bool edge = (kvb + 64 > kv_len) || (p.causal && kvb + 63 > q0 + q_off);
+      const int last = p.causal ? min(kv_len - 1, q_pos + q_off) - kvb : kv_len - 1 - kvb;      // last visible key of the half
+#pragma unroll
+      for (int c = 0; c < 64; c += 32) {
+        uint32_t s[32];
+        tmem_ld32(t_s + c, s);
         tmem_ld_wait();
-        uint32_t dsk[16];
-        // masking is needed only where the block crosses the causal diagonal of this query tile or the end of the keys
-        const bool edge = (kvb + BI > kv_len) || (p.causal && kvb + BI - 1 > q0 + q_off);
 #pragma unroll
         for (int i = 0; i < 32; i += 2) {
-          float dv[2];
-#pragma unroll
-          for (int e = 0; e < 2; ++e) {
-            float pr = fast_exp2(__uint_as_float(s[i + e]) * p.scale_log2 - lse2);
-            if (edge) {
-              const int kv_pos = kvb + c * 32 + i + e;
-              if (kv_pos >= kv_len || (p.causal && kv_pos > q_pos + q_off)) pr = 0.f;
-            }
-            dv[e] = pr * (__uint_as_float(dp[i + e]) - dl);
+          const float2 x = fma2(make_float2(__uint_as_float(s[i]), __uint_as_float(s[i + 1])), scale2, lse_2);
+          float2 pr = make_float2(fast_exp2(x.x), fast_exp2(x.y));
+          if (edge) {
+            if (c + i > last) pr.x = 0.f;
+            if (c + i + 1 > last) pr.y = 0.f;
           }
-          dsk[i >> 1] = pack_bf16(dv[0], dv[1]);
+          const float2 d = mul2(pr, add2(make_float2(__uint_as_float(dp[c + i]), __uint_as_float(dp[c + i + 1])), dl_2));
+          pk[(c + i) >> 1] = pack_bf16(d.x, d.y);
         }
-        tc_fence_before();
-        mbar_arrive(&sd_empty[st]);
-        if (it > 0 && !mbar_wait(acc_done, (it - 1) & 1, p.err, ERR_ATTN_WAIT)) { ok = false; break; }
-        store_row_chunk_sw128(smem + DQ_SMEM_DS, 128, row, c * 32, dsk);
       }
-      fence_proxy_async();
-      mbar_arrive(ds_ready);
+      tmem_st32(t_s, pk);
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(&ds_ready[it & 1]);
     }
-    if (ok && n_iter > 0 && mbar_wait(acc_done, (n_iter - 1) & 1, p.err, ERR_ATTN_WAIT)) {
+    if (ok && n_iter > 0 && mbar_wait(acc_done, 0, p.err, ERR_ATTN_WAIT)) {
       tc_fence_after();
       bf16* dqrow = p.dq + (static_cast<size_t>(seq_start + q_pos) * p.hq + head) * D;
 #pragma unroll 1
@@ -531,22 +591,36 @@ std::vector<torch::Tensor> flash_attn_bwd(const torch::Tensor& dout, const torch
   }
   static bool configured = false;
   if (!configured) {
-    TK_CUDA_CHECK(cudaFuncSetAttribute(flash_bwd_dkdv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fb::KV_SMEM_TOTAL));
-    TK_CUDA_CHECK(cudaFuncSetAttribute(flash_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fb::DQ_SMEM_TOTAL));
+    TK_CUDA_CHECK(cudaFuncSetAttribute(flash_bwd_dkdv_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, fb::SMEM_TOTAL));
+    TK_CUDA_CHECK(cudaFuncSetAttribute(flash_bwd_dkdv_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, fb::SMEM_TOTAL));
+    TK_CUDA_CHECK(cudaFuncSetAttribute(flash_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fb::SMEM_TOTAL));
     configured = true;
   }
   const int tiles = (static_cast<int>(max_seqlen) + fb::BT - 1) / fb::BT;
   const int tiles_k = (static_cast<int>(max_seqlen_k > 0 ? max_seqlen_k : max_seqlen) + fb::BT - 1) / fb::BT;
-  {
-    CUtensorMap tq = make_head_tmap(q, fb::BI), tdo = make_head_tmap(dout, fb::BI), tk_ = make_head_tmap(k, fb::BT), tv = make_head_tmap(v, fb::BT);
-    dim3 grid(hkv, tiles_k, nseq);
-    flash_bwd_dkdv_kernel<<<grid, fb::THREADS, fb::KV_SMEM_TOTAL, stream>>>(tq, tk_, tv, tdo, p);
+  CUtensorMap tq = make_head_tmap(q, fb::BT), tdo = make_head_tmap(dout, fb::BT), tk_ = make_head_tmap(k, fb::BT), tv = make_head_tmap(v, fb::BT);
+  // Where the tiles leave half of the SMs idle, the query heads of a group are shared out over a cluster, as many parts as fit at once (documents of 700
+  // and 324 tokens, 32/8 heads, 72 tiles: 111 us before, 45 with two parts).
+  int parts = 1;
+  const int G = hq / hkv, rows = (static_cast<int>(k.size(0)) + fb::BT - 1) / fb::BT + nseq - 1;      // tiles of all sequences, at most
+  while (parts < 4 && G % (2 * parts) == 0 && 2 * parts * hkv * std::min(rows, tiles_k * nseq) <= num_sms()) parts *= 2;
+  if (parts == 1) {
+    flash_bwd_dkdv_kernel<false><<<dim3(hkv, tiles_k, nseq), fb::THREADS, fb::SMEM_TOTAL, stream>>>(tq, tk_, tv, tdo, p);
+  } else {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(hkv * parts, tiles_k, nseq);
+    cfg.blockDim = dim3(fb::THREADS);
+    cfg.dynamicSmemBytes = fb::SMEM_TOTAL;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = parts;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    TK_CUDA_CHECK(cudaLaunchKernelEx(&cfg, flash_bwd_dkdv_kernel<true>, tq, tk_, tv, tdo, p));
   }
-  {
-    CUtensorMap tq = make_head_tmap(q, fb::BT), tdo = make_head_tmap(dout, fb::BT), tk_ = make_head_tmap(k, fb::BI), tv = make_head_tmap(v, fb::BI);
-    dim3 grid(hq, tiles, nseq);
-    flash_bwd_dq_kernel<<<grid, fb::THREADS, fb::DQ_SMEM_TOTAL, stream>>>(tq, tk_, tv, tdo, p);
-  }
+  flash_bwd_dq_kernel<<<dim3(hq, tiles, nseq), fb::THREADS, fb::SMEM_TOTAL, stream>>>(tq, tk_, tv, tdo, p);
   count_launch(3);
   TK_CUDA_CHECK(cudaGetLastError());
   return {dq, dk, dv};

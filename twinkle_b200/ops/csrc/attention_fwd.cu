@@ -18,6 +18,7 @@
 #include <torch/types.h>
 
 #include "common.cuh"
+#include "elect.cuh"
 #include "host.h"
 #include "scores.cuh"
 
@@ -154,47 +155,51 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     }
   } else if (warp == 9) {
     // ----------------------------------------------------------- MMA issuer
-    if (lane == 0) {
-      constexpr uint32_t idesc_s = umma_idesc_bf16(BQ, BKV, false, false);
-      constexpr uint32_t idesc_o = umma_idesc_bf16(BQ, VA * 64, false, true);
-      const uint32_t sq = smem_u32(smem + S::Q), sp = smem_u32(smem + S::P);
-      auto issue_s = [&](int j) {
-        const uint32_t sk = smem_u32(smem + S::K + (j & 1) * S::K_TILE);
+    // the whole warp walks the loop and one thread issues: inside `if (lane == 0)` each product took 58 ns to issue, as long as it runs
+    constexpr uint32_t idesc_s = umma_idesc_bf16(BQ, BKV, false, false);
+    constexpr uint32_t idesc_o = umma_idesc_bf16(BQ, VA * 64, false, true);
+    const uint64_t dq = umma_desc(smem_u32(smem + S::Q), 16, 1024), dp = umma_desc(smem_u32(smem + S::P), 16, 1024);
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.err, ERR_ATTN_WAIT)); };
+    // addresses in a descriptor count 16 bytes
+    auto issue_s = [&](int j) {
+      const uint64_t dk = umma_desc(smem_u32(smem + S::K + (j & 1) * S::K_TILE), 16, 1024);
+      if (elect_one()) {
 #pragma unroll
         for (int k = 0; k < KA * 4; ++k) {
-          const uint32_t off = (k >> 2) * ATOM_BYTES + (k & 3) * 32;
-          umma_bf16(tmem_base + (j & 1) * 128, umma_desc(sq + off, 16, 1024), umma_desc(sk + off, 16, 1024), idesc_s, k ? 1u : 0u);
+          const uint32_t off = ((k >> 2) * ATOM_BYTES + (k & 3) * 32) >> 4;
+          umma_bf16(tmem_base + (j & 1) * 128, dq + off, dk + off, idesc_s, k ? 1u : 0u);
         }
         umma_commit(&s_full[j & 1]);
-      };
-      bool ok = mbar_wait(q_full, 0, p.err, ERR_ATTN_WAIT) && mbar_wait(&k_full[0], 0, p.err, ERR_ATTN_WAIT);
-      if (ok) {
-        tc_fence_after();
-        issue_s(0);
       }
-      for (int j = 0; ok && j < n_blocks; ++j) {
-        if (j + 1 < n_blocks) {
-          const int n = j + 1;
-          ok = mbar_wait(&k_full[n & 1], (n >> 1) & 1, p.err, ERR_ATTN_WAIT);
-          if (ok && n >= 2) ok = mbar_wait(&s_empty[n & 1], ((n >> 1) - 1) & 1, p.err, ERR_ATTN_WAIT);
-          if (!ok) break;
-          tc_fence_after();
-          issue_s(n);
-        }
-        ok = mbar_wait(p_ready, j & 1, p.err, ERR_ATTN_WAIT) && mbar_wait(&v_full[j % VS], (j / VS) & 1, p.err, ERR_ATTN_WAIT);
+      __syncwarp();
+    };
+    bool ok = wait(q_full, 0) && wait(&k_full[0], 0);
+    if (ok) {
+      tc_fence_after();
+      issue_s(0);
+    }
+    for (int j = 0; ok && j < n_blocks; ++j) {
+      if (j + 1 < n_blocks) {
+        const int n = j + 1;
+        ok = wait(&k_full[n & 1], (n >> 1) & 1);
+        if (ok && n >= 2) ok = wait(&s_empty[n & 1], ((n >> 1) - 1) & 1);
         if (!ok) break;
         tc_fence_after();
-        const uint32_t sv = smem_u32(smem + S::V + (j % VS) * TILE_BYTES);
+        issue_s(n);
+      }
+      ok = wait(p_ready, j & 1) && wait(&v_full[j % VS], (j / VS) & 1);
+      if (!ok) break;
+      tc_fence_after();
+      // A = P (K-major over kv): atom k/4, 32-byte step inside; B = V (MN-major): 16 kv rows = 2048 B per step
+      const uint64_t dv = umma_desc(smem_u32(smem + S::V + (j % VS) * TILE_BYTES), ATOM_BYTES, 1024);
+      if (elect_one()) {
 #pragma unroll
-        for (int k = 0; k < BKV / 16; ++k) {
-          // A = P (K-major over kv): atom k/4, 32-byte step inside; B = V (MN-major): 16 kv rows = 2048 B per step
-          const uint64_t ad = umma_desc(sp + (k >> 2) * ATOM_BYTES + (k & 3) * 32, 16, 1024);
-          const uint64_t bd = umma_desc(sv + k * 2048, ATOM_BYTES, 1024);
-          umma_bf16(tmem_o, ad, bd, idesc_o, (j > 0 || k > 0) ? 1u : 0u);
-        }
+        for (int k = 0; k < BKV / 16; ++k)
+          umma_bf16(tmem_o, dp + (((k >> 2) * ATOM_BYTES + (k & 3) * 32) >> 4), dv + k * (2048 >> 4), idesc_o, k > 0 ? 1u : static_cast<uint32_t>(j > 0));
         umma_commit(o_done);
         umma_commit(&kv_empty[j & 1]);
       }
+      __syncwarp();
     }
   } else {
     // -------------------------------------------------------------- softmax
