@@ -440,3 +440,33 @@ def test_flash_backward_tiles(E, hq, hkv, lens, klens, causal):
     for x, y in zip(got, want):
         assert rel(x, y) < 8e-3        # P and dS rounded to bf16 (2^-9 each at most) and the result too
     assert E.read_and_clear_error() == 0
+
+
+@pytest.mark.parametrize('d,e', [(128, 128), (64, 64), (40, 128), (104, 24)])
+@pytest.mark.parametrize('lens,klens', [((1, 127, 128, 129), None), ((255, 256, 257, 1, 700), None), ((3, 130, 300), (3, 400, 301)), ((400, 260), (100, 300))])
+@pytest.mark.parametrize('window,chunk', [(0, 0), (70, 0), (0, 200), (300, 0)])
+def test_flash_forward_pairs(E, d, e, lens, klens, window, chunk):
+    """Sequences that end in the first or second tile of a pair, keys longer and shorter than their queries, bounds that leave a tile's first blocks unseen."""
+    g = torch.Generator(device='cuda').manual_seed(d + sum(lens))
+    klens, hq, hkv = klens or lens, 6, 2
+    q, k, v = (torch.randn(n, h, w, device='cuda', generator=g).bfloat16() for n, h, w in ((sum(lens), hq, d), (sum(klens), hkv, d), (sum(klens), hkv, e)))
+    cu, cuk = (torch.tensor([0] + list(x), device='cuda').cumsum(0).int() for x in (lens, klens))
+    o, lse = E.flash_attn_fwd(q, k, v, cu, max(lens), True, d ** -0.5, cuk, None, None, window, chunk)
+    a = b = 0
+    for n, m in zip(lens, klens):
+        kk, vv = (t[b:b + m].double().repeat_interleave(hq // hkv, 1) for t in (k, v))
+        s = torch.einsum('qhd,khd->hqk', q[a:a + n].double(), kk) * d ** -0.5
+        i, j = torch.arange(n, device='cuda')[:, None] + m - n, torch.arange(m, device='cuda')[None]
+        seen = j <= i
+        if window:
+            seen &= j > i - window
+        if chunk:
+            seen &= j >= i // chunk * chunk
+        live = seen.any(-1)                        # a query without keys has no defined result
+        s = s.masked_fill(~seen, float('-inf'))
+        want = torch.einsum('hqk,khe->qhe', torch.softmax(s, -1), vv)
+        if live.any():
+            assert rel(o[a:a + n][live], want[live]) < 6e-3            # weights and results rounded to bf16
+            assert (lse[:, a:a + n][:, live].double() - torch.logsumexp(s[:, live], -1)).abs().max() < 5e-3
+        a, b = a + n, b + m
+    assert E.read_and_clear_error() == 0

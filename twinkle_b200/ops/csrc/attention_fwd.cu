@@ -5,12 +5,14 @@
 // formed once per tile, one per softmax thread), and a last chunk of key dimensions that all heads share (rotated part of latent attention), loaded from a tensor of
 // its own so that nothing has to put the keys together.
 //
-// One CTA per (128-row query tile of one sequence, query head).  192 threads:
-//   warps 0-3  softmax: thread = one query row; reads S from tensor memory (tcgen05.ld), keeps the
+// Keys of up to two chunks without score terms take two query tiles per CTA (flash_fwd_pair_kernel below); the kernel described here is for the rest.
+//
+// One CTA per (128-row query tile of one sequence, query head).  320 threads:
+//   warps 0-7  softmax: thread = one query row; reads S from tensor memory (tcgen05.ld), keeps the
 //              running max / sum, writes P (bf16) into a 128-byte-swizzled smem tile, rescales the O
 //              accumulator in tensor memory only when a row maximum grows by more than 2^8
-//   warp 4     TMA producer: Q once, then K/V tiles (double buffered)
-//   warp 5     MMA issuer: S_j = Q·K_jᵀ into one of two TMEM buffers (so S_{j+1} is computed while
+//   warp 8     TMA producer: Q once, then K/V tiles (double buffered)
+//   warp 9     MMA issuer: S_j = Q·K_jᵀ into one of two TMEM buffers (so S_{j+1} is computed while
 //              the softmax of S_j runs), O += P_j·V_j into a third TMEM buffer
 // Tensor memory: S0 [0,128), S1 [128,256), O [256,384) fp32 columns.
 #include <ATen/cuda/CUDAContext.h>
@@ -61,6 +63,47 @@ struct FwdParams {
   int tail_col;       // first column of a query row that meets the shared part
   int* err;
 };
+
+// Columns [32·c0, 32·c1) of a finished row of the output, from its TMEM lane.
+template <int VA>
+__device__ __forceinline__ void store_out(const FwdParams& p, uint32_t tmem_row, int head, int token, bool valid, float inv_l, int c0, int c1) {
+  const bf16* gate = p.gate.p != nullptr && valid ? reinterpret_cast<const bf16*>(p.gate.p) + static_cast<size_t>(token) * p.gate.ld + static_cast<size_t>(head) * max(p.gate.e, 1) : nullptr;
+  if (gate != nullptr && p.gate.e == 0) inv_l *= sigmoid_of(__bfloat162float(*gate));
+  bf16* orow = p.out + (static_cast<size_t>(token) * p.hq + head) * p.e;
+#pragma unroll 1
+  for (int c = c0; c < c1 && c * 32 < p.e; ++c) {
+    uint32_t r[32];
+    tmem_ld32(tmem_row + c * 32, r);
+    tmem_ld_wait();
+    if (valid) {
+#pragma unroll
+      for (int i = 0; i < 32; i += 8) {
+        if (VA == 1 || c >= 2) { if (c * 32 + i >= p.e) break; }
+        if (gate != nullptr && p.gate.e > 0) {
+          if (p.gate_vec) {
+            const uint4 g = *reinterpret_cast<const uint4*>(gate + c * 32 + i);
+            const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+              const float2 z = unpack_bf16(gw[x]);
+              r[i + 2 * x] = __float_as_uint(__uint_as_float(r[i + 2 * x]) * sigmoid_of(z.x));
+              r[i + 2 * x + 1] = __float_as_uint(__uint_as_float(r[i + 2 * x + 1]) * sigmoid_of(z.y));
+            }
+          } else {
+#pragma unroll
+            for (int x = 0; x < 8; ++x)
+              if (c * 32 + i + x < p.gate.e) r[i + x] = __float_as_uint(__uint_as_float(r[i + x]) * sigmoid_of(__bfloat162float(gate[c * 32 + i + x])));
+          }
+        }
+        uint4 v = make_uint4(pack_bf16(__uint_as_float(r[i]) * inv_l, __uint_as_float(r[i + 1]) * inv_l),
+                             pack_bf16(__uint_as_float(r[i + 2]) * inv_l, __uint_as_float(r[i + 3]) * inv_l),
+                             pack_bf16(__uint_as_float(r[i + 4]) * inv_l, __uint_as_float(r[i + 5]) * inv_l),
+                             pack_bf16(__uint_as_float(r[i + 6]) * inv_l, __uint_as_float(r[i + 7]) * inv_l));
+        *reinterpret_cast<uint4*>(orow + c * 32 + i) = v;
+      }
+    }
+  }
+}
 
 // KA / VA: 64-wide chunks of a query / key row (up to 3) and of a value row (1 or 2).
 template <int KA, int VA, bool TERMS>
@@ -334,46 +377,256 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     if (!dead && n_blocks > 0 && mbar_wait(o_done, (n_blocks - 1) & 1, p.err, ERR_ATTN_WAIT)) {
       tc_fence_after();
       if (p.sinks != nullptr) l_sum += exp2f(__bfloat162float(p.sinks[head]) * 1.4426950408889634f - m_used);
-      float inv_l = (l_sum > 0.f) ? 1.f / l_sum : 0.f;
       const bool valid = q_pos < seq_len;
-      const bf16* gate = p.gate.p != nullptr && valid ? reinterpret_cast<const bf16*>(p.gate.p) + static_cast<size_t>(seq_start + q_pos) * p.gate.ld + static_cast<size_t>(head) * max(p.gate.e, 1)
-                                                      : nullptr;
-      if (gate != nullptr && p.gate.e == 0) inv_l *= sigmoid_of(__bfloat162float(*gate));
-      bf16* orow = p.out + (static_cast<size_t>(seq_start + q_pos) * p.hq + head) * p.e;
-#pragma unroll 1
-      for (int c = 2 * wg; c < 2 * wg + 2 && c * 32 < p.e; ++c) {
-        uint32_t r[32];
-        tmem_ld32(tmem_o + lane_off + c * 32, r);
-        tmem_ld_wait();
-        if (valid) {
-#pragma unroll
-          for (int i = 0; i < 32; i += 8) {
-            if (VA == 1 || c >= 2) { if (c * 32 + i >= p.e) break; }
-            if (gate != nullptr && p.gate.e > 0) {
-              if (p.gate_vec) {
-                const uint4 g = *reinterpret_cast<const uint4*>(gate + c * 32 + i);
-                const uint32_t gw[4] = {g.x, g.y, g.z, g.w};
-#pragma unroll
-                for (int x = 0; x < 4; ++x) {
-                  const float2 z = unpack_bf16(gw[x]);
-                  r[i + 2 * x] = __float_as_uint(__uint_as_float(r[i + 2 * x]) * sigmoid_of(z.x));
-                  r[i + 2 * x + 1] = __float_as_uint(__uint_as_float(r[i + 2 * x + 1]) * sigmoid_of(z.y));
-                }
-              } else {
-#pragma unroll
-                for (int x = 0; x < 8; ++x)
-                  if (c * 32 + i + x < p.gate.e) r[i + x] = __float_as_uint(__uint_as_float(r[i + x]) * sigmoid_of(__bfloat162float(gate[c * 32 + i + x])));
-              }
-            }
-            uint4 v = make_uint4(pack_bf16(__uint_as_float(r[i]) * inv_l, __uint_as_float(r[i + 1]) * inv_l),
-                                 pack_bf16(__uint_as_float(r[i + 2]) * inv_l, __uint_as_float(r[i + 3]) * inv_l),
-                                 pack_bf16(__uint_as_float(r[i + 4]) * inv_l, __uint_as_float(r[i + 5]) * inv_l),
-                                 pack_bf16(__uint_as_float(r[i + 6]) * inv_l, __uint_as_float(r[i + 7]) * inv_l));
-            *reinterpret_cast<uint4*>(orow + c * 32 + i) = v;
-          }
-        }
-      }
+      store_out<VA>(p, tmem_o + lane_off, head, seq_start + q_pos, valid, (l_sum > 0.f) ? 1.f / l_sum : 0.f, 2 * wg, 2 * wg + 2);
       if (valid && wg == 0) p.lse[static_cast<size_t>(head) * p.T + seq_start + q_pos] = (m_used + log2f(l_sum)) * 0.6931471805599453f;
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 9) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+// Two query tiles per CTA, for keys of up to two chunks without score terms.
+//
+// One tile at a time leaves the tensor cores idle while its softmax runs and the other way round (420 TFLOP/s).  Here warps 0-3 and 4-7 have a tile
+// each, a thread a whole row, and the products of one tile run under the softmax of the other; P goes into the TMEM columns of its scores, as
+// the A operand of the second product.  Keys and values are loaded once for both tiles.  Every row is computed with the same operations in
+// the same order as in the kernel above (the sum of P in two halves), so the results are the same to the bit.
+// 32/8 heads of 128, causal, us before → now: 8192 tokens 1177 → 540 (1020 TFLOP/s; what is left is the exponentials, 1024 cycles of a block on
+// the special-function units against 1024 of its products), 8 x 1024 258 → 137, 700 + 324 33 → 23; 32/4 heads, 8 x 4096 2590 → 1207.
+// Tensor memory: S [0,128) and [128,256), P in the first 64 columns of its S, O [256,384) and [384,512).
+namespace fa2 {
+constexpr int Q = 0, K = 4 * fa::ATOM_BYTES, V = K + 2 * fa::TILE_BYTES, BAR = V + 2 * fa::TILE_BYTES, TOTAL = BAR + 256 + 1024;
+}
+
+template <int KA, int VA>
+__global__ void __launch_bounds__(fa::THREADS, 1)
+flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
+                      const __grid_constant__ CUtensorMap tmR, const FwdParams p) {
+  using namespace fa;
+  const int head = blockIdx.x, seq = blockIdx.z;
+  const int seq_start = p.cu[seq], seq_len = p.cu[seq + 1] - seq_start;
+  const int n_pairs = (seq_len + 2 * BQ - 1) / (2 * BQ);
+  if (static_cast<int>(blockIdx.y) >= n_pairs) return;
+  const int q0 = (n_pairs - 1 - blockIdx.y) * 2 * BQ;              // longest first
+  const int kv_head = head / (p.hq / p.hkv);
+  const int kv_start = p.cu_k[seq], kv_len = p.cu_k[seq + 1] - kv_start;
+  const int q_off = kv_len - seq_len;
+  const bool bounded = p.window > 0 || p.chunk > 0;
+  const int jb0 = bounded ? first_visible(max(q0 + q_off, 0), p.window, p.chunk) / BKV : 0;
+  auto end_of = [&](int t) { return q0 + t * BQ >= seq_len ? 0 : p.causal ? max(0, min(kv_len, q0 + (t + 1) * BQ + q_off)) : kv_len; };
+  auto blocks_of = [&](int t) { return max(0, (end_of(t) + BKV - 1) / BKV - jb0); };
+  const int n_a = blocks_of(0), n_b = blocks_of(1), n_all = max(n_a, n_b);
+
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + fa2::BAR);
+  uint64_t* q_full = bars;            // 1
+  uint64_t* k_full = bars + 1;        // 2 stages each
+  uint64_t* k_empty = bars + 3;
+  uint64_t* v_full = bars + 5;
+  uint64_t* v_empty = bars + 7;
+  uint64_t* s_full = bars + 9;        // 2 tiles each
+  uint64_t* p_ready = bars + 11;
+  uint64_t* o_done = bars + 13;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 15);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    mbar_init(q_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&k_full[i], 1);
+      mbar_init(&k_empty[i], 1);
+      mbar_init(&v_full[i], 1);
+      mbar_init(&v_empty[i], 1);
+      mbar_init(&s_full[i], 1);
+      mbar_init(&p_ready[i], 128);
+      mbar_init(&o_done[i], 1);
+    }
+    fence_barrier_init();
+  }
+  if (warp == 9) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(tmem_slot);
+
+  if (warp == 8) {
+    // ------------------------------------------------------------- producer
+    if (lane == 0 && n_all > 0) {
+      tma_prefetch_desc(&tmQ);
+      tma_prefetch_desc(&tmK);
+      tma_prefetch_desc(&tmV);
+      mbar_expect_tx(q_full, 2 * KA * ATOM_BYTES);      // rows past the tensor arrive as zeros, those of the next sequence are not stored
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int c = 0; c < KA; ++c)
+          tma_load_3d(smem + fa2::Q + (t * KA + c) * ATOM_BYTES, &tmQ, q_full, c < p.own_chunks ? c * 64 : p.tail_col, head, seq_start + q0 + t * BQ);
+      for (int j = 0; j < n_all; ++j) {
+        const int st = j & 1, row = kv_start + (jb0 + j) * BKV;
+        if (j >= 2 && !mbar_wait(&k_empty[st], ((j >> 1) - 1) & 1, p.err, ERR_ATTN_WAIT)) break;
+        mbar_expect_tx(&k_full[st], KA * ATOM_BYTES);
+#pragma unroll
+        for (int c = 0; c < KA; ++c) {
+          uint8_t* dst = smem + fa2::K + st * TILE_BYTES + c * ATOM_BYTES;
+          if (c < p.own_chunks) tma_load_3d(dst, &tmK, &k_full[st], c * 64, kv_head, row);
+          else tma_load_3d(dst, &tmR, &k_full[st], 0, 0, row);
+        }
+        if (j >= 2 && !mbar_wait(&v_empty[st], ((j >> 1) - 1) & 1, p.err, ERR_ATTN_WAIT)) break;
+        mbar_expect_tx(&v_full[st], VA * ATOM_BYTES);
+#pragma unroll
+        for (int c = 0; c < VA; ++c) tma_load_3d(smem + fa2::V + st * TILE_BYTES + c * ATOM_BYTES, &tmV, &v_full[st], c * 64, kv_head, row);
+      }
+    }
+  } else if (warp == 9) {
+    // ----------------------------------------------------------- MMA issuer
+    constexpr uint32_t idesc_s = umma_idesc_bf16(BQ, BKV, false, false);
+    constexpr uint32_t idesc_o = umma_idesc_bf16(BQ, VA * 64, false, true);
+    const uint64_t dq = umma_desc(smem_u32(smem + fa2::Q), 16, 1024);
+    auto wait = [&](uint64_t* bar, uint32_t parity) { return __all_sync(0xffffffffu, mbar_wait(bar, parity, p.err, ERR_ATTN_WAIT)); };
+    auto scores = [&](int t, int j) {
+      const uint64_t dk = umma_desc(smem_u32(smem + fa2::K + (j & 1) * TILE_BYTES), 16, 1024), q = dq + t * (KA * ATOM_BYTES >> 4);
+      if (elect_one()) {
+#pragma unroll
+        for (int k = 0; k < KA * 4; ++k) {
+          const uint32_t off = ((k >> 2) * ATOM_BYTES + (k & 3) * 32) >> 4;
+          umma_bf16(tmem_base + t * 128, q + off, dk + off, idesc_s, k ? 1u : 0u);
+        }
+        umma_commit(&s_full[t]);
+      }
+      __syncwarp();
+    };
+    auto commit = [&](uint64_t* bar) {
+      if (elect_one()) umma_commit(bar);
+      __syncwarp();
+    };
+    bool ok = n_all > 0 && wait(q_full, 0) && wait(&k_full[0], 0);
+    if (ok) {
+      tc_fence_after();
+      if (n_a > 0) scores(0, 0);
+      if (n_b > 0) scores(1, 0);
+      commit(&k_empty[0]);
+    }
+    for (int j = 0; ok && j < n_all; ++j) {
+      const uint64_t dv = umma_desc(smem_u32(smem + fa2::V + (j & 1) * TILE_BYTES), ATOM_BYTES, 1024);
+      if (!wait(&v_full[j & 1], (j >> 1) & 1)) break;
+      if (j + 1 < n_all && !wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1)) break;
+#pragma unroll 1
+      for (int t = 0; t < 2; ++t) {
+        const int n = t == 0 ? n_a : n_b;
+        if (j >= n) continue;
+        ok = wait(&p_ready[t], j & 1);
+        if (!ok) break;
+        tc_fence_after();
+        if (elect_one()) {
+#pragma unroll
+          for (int k = 0; k < BKV / 16; ++k)
+            umma_bf16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + k * 8, dv + k * (2048 >> 4), idesc_o, k > 0 ? 1u : static_cast<uint32_t>(j > 0));
+          if (j == n - 1) umma_commit(&o_done[t]);
+        }
+        __syncwarp();
+        if (j + 1 < n) scores(t, j + 1);                 // runs after the product that reads P from the same columns
+      }
+      commit(&v_empty[j & 1]);
+      if (j + 1 < n_all) commit(&k_empty[(j + 1) & 1]);
+    }
+  } else {
+    // -------------------------------------------------------------- softmax
+    const int t = warp >> 2, qt = q0 + t * BQ, n_blocks = t == 0 ? n_a : n_b, kv_end = end_of(t);
+    const int row = (warp & 3) * 32 + lane, q_pos = qt + row;
+    const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
+    const uint32_t ts = tmem_base + t * 128 + lane_off, to = tmem_base + 256 + t * 128 + lane_off;
+    const int first = bounded ? first_visible(max(q_pos + q_off, 0), p.window, p.chunk) : 0;
+    const int first_last = bounded ? first_visible(max(qt + BQ - 1 + q_off, 0), p.window, p.chunk) : 0;
+    const float2 scale2 = make_float2(p.scale_log2, p.scale_log2);
+    float m_used = -INFINITY;
+    float2 l2 = make_float2(0.f, 0.f);       // sums over the first and second 64 keys of the blocks
+    bool dead = false;
+    for (int j = 0; j < n_blocks; ++j) {
+      if (!mbar_wait(&s_full[t], j & 1, p.err, ERR_ATTN_WAIT)) { dead = true; break; }
+      tc_fence_after();
+      float sc[128];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) tmem_ld32(ts + c * 32, *reinterpret_cast<uint32_t(*)[32]>(sc + c * 32));
+      tmem_ld_wait();
+      const int kv0 = (jb0 + j) * BKV;
+#pragma unroll
+      for (int i = 0; i < 128; i += 2) {
+        const float2 x = mul2(make_float2(sc[i], sc[i + 1]), scale2);
+        sc[i] = x.x;
+        sc[i + 1] = x.y;
+      }
+      if ((kv0 + BKV > kv_end) || (p.causal && kv0 + BKV > qt + q_off) || kv0 < first_last) {
+        const int last = (p.causal ? min(kv_end - 1, q_pos + q_off) : kv_end - 1) - kv0, begin = first - kv0;
+#pragma unroll
+        for (int i = 0; i < 128; ++i)
+          if (i > last || i < begin) sc[i] = -INFINITY;
+      }
+      float mx4[4] = {sc[0], sc[1], sc[2], sc[3]};
+#pragma unroll
+      for (int i = 4; i < 128; i += 4) {
+        mx4[0] = fmaxf(mx4[0], sc[i]);
+        mx4[1] = fmaxf(mx4[1], sc[i + 1]);
+        mx4[2] = fmaxf(mx4[2], sc[i + 2]);
+        mx4[3] = fmaxf(mx4[3], sc[i + 3]);
+      }
+      const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
+      float alpha = 1.f;
+      bool rescale = false;
+      // a row may see none of its first blocks: its maximum then stays at −∞ and its weights are zero
+      if (mx > m_used + RESCALE_THRESHOLD || (m_used == -INFINITY && mx != -INFINITY)) {
+        alpha = (m_used == -INFINITY) ? 0.f : exp2f(m_used - mx);
+        rescale = (j > 0);
+        m_used = mx;
+        l2.x *= alpha;
+        l2.y *= alpha;
+      }
+      const float m_sub = m_used == -INFINITY ? 0.f : m_used;
+      // the product that added the block before has retired: it was issued ahead of these scores
+      if (__any_sync(0xffffffffu, rescale)) {
+#pragma unroll 1
+        for (int c = 0; c < 2 * VA; ++c) {
+          uint32_t r[32];
+          tmem_ld32(to + c * 32, r);
+          tmem_ld_wait();
+#pragma unroll
+          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * alpha);
+          tmem_st32(to + c * 32, r);
+        }
+        tmem_st_wait();
+      }
+      const float2 neg = make_float2(-m_sub, -m_sub);
+      uint32_t pa[32], pb[32];
+#pragma unroll
+      for (int i = 0; i < 64; i += 2) {
+        const float2 x = add2(make_float2(sc[i], sc[i + 1]), neg), y = add2(make_float2(sc[64 + i], sc[64 + i + 1]), neg);
+        pa[i >> 1] = pack_bf16(fast_exp2(x.x), fast_exp2(x.y));
+        pb[i >> 1] = pack_bf16(fast_exp2(y.x), fast_exp2(y.y));
+        // the sum uses the bf16-rounded values so that numerator and denominator match
+        const float2 u = unpack_bf16(pa[i >> 1]), v = unpack_bf16(pb[i >> 1]);
+        l2 = add2(l2, add2(make_float2(u.x, v.x), make_float2(u.y, v.y)));
+      }
+      tmem_st32(ts, pa);
+      tmem_st32(ts + 32, pb);
+      tmem_st_wait();
+      tc_fence_before();
+      mbar_arrive(&p_ready[t]);
+    }
+    // ------------------------------------------------------------- epilogue
+    if (!dead && n_blocks > 0 && mbar_wait(&o_done[t], 0, p.err, ERR_ATTN_WAIT)) {
+      tc_fence_after();
+      float l_sum = l2.x + l2.y;
+      if (p.sinks != nullptr) l_sum += exp2f(__bfloat162float(p.sinks[head]) * 1.4426950408889634f - m_used);
+      const bool valid = q_pos < seq_len;
+      store_out<VA>(p, to, head, seq_start + q_pos, valid, (l_sum > 0.f) ? 1.f / l_sum : 0.f, 0, 2 * VA);
+      if (valid) p.lse[static_cast<size_t>(head) * p.T + seq_start + q_pos] = (m_used + log2f(l_sum)) * 0.6931471805599453f;
     }
   }
   tc_fence_before();
@@ -435,7 +688,6 @@ std::vector<torch::Tensor> flash_attn_fwd(const torch::Tensor& q, const torch::T
   p.window = window; p.chunk = chunk; p.own_chunks = own_chunks; p.tail_col = k.size(2);
   const dim3 grid(hq, (static_cast<int>(max_seqlen) + fa::BQ - 1) / fa::BQ, nseq);
   auto stream = at::cuda::getCurrentCUDAStream();
-#define TK_FLASH(KA, VA) do { if (p.terms.used) TK_FLASH_RUN(KA, VA, true); else TK_FLASH_RUN(KA, VA, false); } while (0)
 #define TK_FLASH_RUN(KA, VA, TERMS)                                                                                                     \
   do {                                                                                                                                  \
     static bool configured = false;                                                                                                     \
@@ -446,13 +698,35 @@ std::vector<torch::Tensor> flash_attn_fwd(const torch::Tensor& q, const torch::T
     flash_fwd_kernel<KA, VA, TERMS><<<grid, fa::THREADS, fa::Smem<KA>::TOTAL, stream>>>(tq, tk_, tv, tr, p);                                   \
   } while (0)
   const bool wide_k = chunks > 1, wide_v = v.size(2) > 64;
-  if (chunks == 3 && wide_v) TK_FLASH(3, 2);
-  else if (chunks == 3) TK_FLASH(3, 1);
-  else if (wide_k && wide_v) TK_FLASH(2, 2);
-  else if (wide_k) TK_FLASH(2, 1);
-  else if (wide_v) TK_FLASH(1, 2);
-  else TK_FLASH(1, 1);
-#undef TK_FLASH
+  // two tiles per CTA wherever their keys fit shared memory, at every size: 16/8 heads, one prompt of 16 tokens 9.7 → 8.1 us, 448 17.4 → 16.3
+  const bool pairs = chunks <= 2 && !p.terms.used;
+  if (pairs) {
+    const dim3 half(hq, (grid.y + 1) / 2, nseq);
+    auto go = [&](auto kern, bool& configured) {
+      if (!configured) {
+        TK_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fa2::TOTAL));
+        configured = true;
+      }
+      kern<<<half, fa::THREADS, fa2::TOTAL, stream>>>(tq, tk_, tv, tr, p);
+    };
+    static bool configured[4];
+    if (wide_k && wide_v) go(flash_fwd_pair_kernel<2, 2>, configured[0]);
+    else if (wide_k) go(flash_fwd_pair_kernel<2, 1>, configured[1]);
+    else if (wide_v) go(flash_fwd_pair_kernel<1, 2>, configured[2]);
+    else go(flash_fwd_pair_kernel<1, 1>, configured[3]);
+    count_launch();
+    TK_CUDA_CHECK(cudaGetLastError());
+    return {out, lse};
+  }
+  if (chunks == 3 && !p.terms.used) {
+    if (wide_v) TK_FLASH_RUN(3, 2, false); else TK_FLASH_RUN(3, 1, false);
+  } else if (chunks == 3) {
+    if (wide_v) TK_FLASH_RUN(3, 2, true); else TK_FLASH_RUN(3, 1, true);
+  } else if (wide_k) {
+    if (wide_v) TK_FLASH_RUN(2, 2, true); else TK_FLASH_RUN(2, 1, true);
+  } else {
+    if (wide_v) TK_FLASH_RUN(1, 2, true); else TK_FLASH_RUN(1, 1, true);
+  }
 #undef TK_FLASH_RUN
   count_launch();
   TK_CUDA_CHECK(cudaGetLastError());
