@@ -470,3 +470,28 @@ def test_flash_forward_pairs(E, d, e, lens, klens, window, chunk):
             assert (lse[:, a:a + n][:, live].double() - torch.logsumexp(s[:, live], -1)).abs().max() < 5e-3
         a, b = a + n, b + m
     assert E.read_and_clear_error() == 0
+
+
+@pytest.mark.parametrize('dtype,hkv,d,e', [(torch.bfloat16, 8, 128, 128), (torch.bfloat16, 1, 24, 40), (torch.float32, 3, 64, 4), (torch.bfloat16, 1, 4, 3)])
+@pytest.mark.parametrize('lens', [(1, ), (16, 1, 17), (300, 37, 111)])
+def test_cache_write_places(E, dtype, hkv, d, e, lens):
+    """Rows of prompts land where their block lists say and nowhere else: whole vectors, narrow rows (the general path), views with a pitch of their own."""
+    from twinkle_b200 import ops
+    bs, T = 16, sum(lens)
+    need = [(n + bs - 1) // bs for n in lens]
+    perm = (torch.randperm(sum(need)) + 1).tolist()
+    blocks = [[perm.pop() for _ in range(n)] for n in need]
+    rows = E.prompt_rows(blocks, list(lens), bs, True).cuda()
+    kp, vp = (torch.zeros(sum(need) + 2, bs, hkv, w, device='cuda', dtype=dtype) for w in (d, e))
+    both = torch.randn(T, hkv * (d + e) + 8, device='cuda').to(dtype)
+    k, v = both[:, :hkv * d].view(T, hkv, d), both[:, hkv * d:hkv * (d + e)].view(T, hkv, e)
+    ops.cache_write(kp, vp, rows, k, v)
+    want_k, want_v, at = torch.zeros_like(kp), torch.zeros_like(vp), 0
+    for n, b in zip(lens, blocks):
+        for t in range(n):
+            want_k[b[t // bs], t % bs], want_v[b[t // bs], t % bs] = k[at + t], v[at + t]
+        at += n
+    assert torch.equal(kp, want_k) and torch.equal(vp, want_v)
+    out = torch.full((4 * (5 + 2), ), -1, dtype=torch.int32)
+    E.pack_step(out, 4, 5, [[7, 8, 9], [3]], [40, 2], [1, 2])
+    assert out.tolist() == [7, 8, 9, 0, 0, 3, 0, 0, 0, 0] + [0] * 10 + [40, 2, 0, 0] + [1, 2, 0, 0]

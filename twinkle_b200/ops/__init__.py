@@ -816,6 +816,16 @@ def paged_attention_decode(q, k_cache, v_cache, block_tables, seq_lens, scale: O
     return _open_gate(ref.paged_attention_decode(q, k_cache, v_cache, block_tables, seq_lens, scale, window, softcap, sinks, chunk, terms), gate)
 
 
+def cache_write(k_pool, v_pool, rows, k, v) -> None:
+    """Store ``k, v [T, heads, width]`` in rows ``rows [T]`` (block · block size + offset) of the paged pools ``[blocks, block size, heads, width]``."""
+    if _cuda(k) and all(p.dtype == x.dtype and p.shape[2:] == x.shape[1:] and p.is_contiguous() and x.shape[1] * x.shape[2] * x.element_size() % 16 == 0
+                        and x.stride(2) == 1 and x.stride(1) == x.shape[2] and x.stride(0) * x.element_size() % 16 == 0 and x.data_ptr() % 16 == 0 and p.data_ptr() % 16 == 0
+                        for p, x in ((k_pool, k), (v_pool, v))):
+        return ext().cache_write(k_pool, v_pool, rows, k, v)
+    for p, x in ((k_pool, k), (v_pool, v)):
+        p.view(-1, *p.shape[2:])[rows] = x
+
+
 # ------------------------------------------------------ gated delta net (linear attention)
 def _segment_starts(cu_seqlens: torch.Tensor, total: int) -> torch.Tensor:
     """``[T]`` int32: for every packed token the index of the first token of its sequence."""

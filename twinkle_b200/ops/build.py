@@ -25,7 +25,7 @@ _HERE = os.path.dirname(os.path.abspath(__file__))
 _CSRC = os.path.join(_HERE, 'csrc')
 _SO = os.path.join(_HERE, '_C.so')
 _STAMP = os.path.join(_HERE, '_C.stamp')
-_SERVING_SOURCES = ('bindings.cpp', 'host.cu', 'gemm.cu', 'gemm2.cu', 'gemm_skinny.cu', 'attention_fwd.cu', 'attention_packed.cu', 'decode.cu', 'paged_decode.cu', 'sample.cu', 'stream_ops.cu')
+_SERVING_SOURCES = ('bindings.cpp', 'host.cu', 'gemm.cu', 'gemm2.cu', 'gemm_skinny.cu', 'attention_fwd.cu', 'attention_packed.cu', 'cache_write.cu', 'decode.cu', 'paged_decode.cu', 'sample.cu', 'stream_ops.cu')
 # mechanism → its sources (``DecoderConfig.kernel_parts`` names those a model has)
 _PARTS = {'convolution': ('conv_heads.cu', ), 'experts': ('moe_serve.cu', ), 'heads': ('heads.cu', ), 'latent': ('latent.cu', 'latent_decode.cu'), 'memory': ('mlstm.cu', ),
           'recurrent': ('hgrn2.cu', ), 'rotary': ('rotary.cu', ), 'selective': ('selective.cu', )}

@@ -15,6 +15,9 @@ torch::Tensor attention_packed(const torch::Tensor&, const torch::Tensor&, const
                                const c10::optional<torch::Tensor>&, const c10::optional<torch::Tensor>&, int64_t, int64_t, double, const c10::optional<torch::Tensor>&, const c10::optional<torch::Tensor>&, const c10::optional<torch::Tensor>&, const c10::optional<torch::Tensor>&, const c10::optional<torch::Tensor>&);
 torch::Tensor paged_attn_decode(const torch::Tensor&, const torch::Tensor&, const torch::Tensor&, const torch::Tensor&, const torch::Tensor&, double, int64_t, int64_t,
                                 const c10::optional<torch::Tensor>&, const c10::optional<torch::Tensor>&, double, const c10::optional<torch::Tensor>&, const c10::optional<torch::Tensor>&, const c10::optional<torch::Tensor>&, const c10::optional<torch::Tensor>&, const c10::optional<torch::Tensor>&);
+void cache_write(const torch::Tensor&, const torch::Tensor&, const torch::Tensor&, const torch::Tensor&, const torch::Tensor&);
+void pack_step(const torch::Tensor&, int64_t, int64_t, const std::vector<std::vector<int32_t>>&, const std::vector<int32_t>&, const std::vector<int32_t>&);
+torch::Tensor prompt_rows(const std::vector<std::vector<int32_t>>&, const std::vector<int64_t>&, int64_t, bool);
 std::vector<torch::Tensor> sample_tokens(const torch::Tensor&, double, int64_t, double, const torch::Tensor&);
 std::vector<torch::Tensor> conv_heads(const torch::Tensor&, const c10::optional<torch::Tensor>&, const torch::Tensor&, int64_t, int64_t, int64_t, int64_t,
                                       double, double, int64_t, const c10::optional<torch::Tensor>&, const c10::optional<torch::Tensor>&, bool,
@@ -128,6 +131,9 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("paged_attn_decode", &tk::paged_attn_decode, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("tables"), py::arg("seq_lens"), py::arg("scale"),
         py::arg("window") = 0, py::arg("chunk") = 0, py::arg("sinks") = py::none(), py::arg("gate") = py::none(), py::arg("cap") = 0.0, py::arg("temp") = py::none(), py::arg("slope") = py::none(),
         py::arg("rate") = py::none(), py::arg("table") = py::none(), py::arg("bucket") = py::none());
+  m.def("cache_write", &tk::cache_write);
+  m.def("pack_step", &tk::pack_step);
+  m.def("prompt_rows", &tk::prompt_rows);
   m.def("sample_tokens", &tk::sample_tokens);
   m.def("set_gemm_pair", &tk::set_gemm_pair);
   m.def("set_gemm_staged", &tk::set_gemm_staged);

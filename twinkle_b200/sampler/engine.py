@@ -175,6 +175,13 @@ class NativeEngine:
             self.cache.release_slot(s.state_slot)
             s.blocks, s.state_slot, s.linear = [], 0, {}
 
+    def _prompt_rows(self, seqs: Sequence[_Seq], lens: Sequence[int]) -> torch.Tensor:
+        """Rows of the cache pools for packed prompts ``[ΣL]``, listed on the host and copied once."""
+        bs = self.cache.block_size
+        if self.device.type == 'cuda':
+            return ops.ext().prompt_rows([s.blocks for s in seqs], lens, bs, True).to(self.device, non_blocking=True)
+        return torch.tensor([s.blocks[p // bs] * bs + p % bs for s, n in zip(seqs, lens) for p in range(n)], dtype=torch.int64, device=self.device)
+
     def _prompt_view(self, seqs: Sequence[_Seq], lens: Sequence[int]) -> CacheView:
         """Cache places of packed prompts: one row per token, built on the host and copied once."""
         bs = self.cache.block_size
@@ -194,13 +201,17 @@ class NativeEngine:
         lens = [len(s.prompt) for s in seqs]
         ids = torch.tensor([t for s in seqs for t in s.prompt], dtype=torch.long, device=self.device)
         pos = torch.cat([torch.arange(n, device=self.device) for n in lens])
-        cu = torch.tensor([0] + list(torch.tensor(lens).cumsum(0)), dtype=torch.int32, device=self.device)
+        bounds = [0]
+        for n in lens:
+            bounds.append(bounds[-1] + n)
+        cu = torch.tensor(bounds, dtype=torch.int32, device=self.device)
         self.admit(seqs)
-        bounds = cu.tolist()
+        rows: List[torch.Tensor] = []       # places of all tokens, when a layer wants them
 
         def sink(layer: int, k: torch.Tensor, v: torch.Tensor) -> None:
-            for s, a, b in zip(seqs, bounds[:-1], bounds[1:]):
-                self.cache.write(layer, s.blocks, 0, k[a:b], v[a:b])
+            if not rows:
+                rows.append(self._prompt_rows(seqs, lens))
+            ops.cache_write(self.cache.k[layer], self.cache.v[layer], rows[0], k, v)
 
         def linear_state(layer: int, conv: torch.Tensor, state: torch.Tensor) -> None:  # hybrid stacks: what decode continues from
             for i, s in enumerate(seqs):
@@ -252,8 +263,8 @@ class NativeEngine:
         if cfg.rope_local_theta:       # sliding-window layers of Gemma-3 rotate with a base of their own
             local = ops.rope_tables(positions if rope_positions is None else rope_positions, cfg.rotary_dim, cfg.rope_local_theta, None)
         x = self.model.embed_ids(tokens)
-        blk = table.gather(1, (positions // self.cache.block_size).unsqueeze(1)).squeeze(1).long()
-        off = positions % self.cache.block_size
+        bs = self.cache.block_size
+        rows = table.gather(1, (positions // bs).unsqueeze(1)).squeeze(1).long() * bs + positions % bs
         with lora_batch(lora):
             for li, layer in enumerate(self.model.layers):
                 at = layer.self_attn
@@ -268,7 +279,7 @@ class NativeEngine:
                     x = x + layer.feed_forward(n)
                     continue
                 q, k, v, gate = at.heads_from(h, *(local if (local is not None and getattr(at, 'local_rope', False)) else (cos, sin)))
-                self.cache.k[li][blk, off], self.cache.v[li][blk, off] = at.cache_entry(k, v)
+                ops.cache_write(self.cache.k[li], self.cache.v[li], rows, *at.cache_entry(k, v))
                 o = ops.paged_attention_decode(q, self.cache.k[li], self.cache.v[li], table, seq_lens, at.scale,
                                                window=getattr(at, 'window', None), softcap=getattr(at, 'softcap', None), sinks=getattr(at, 'sinks', None))
                 n, x = layer.after_attention(x, at.project_out(o, gate))
@@ -285,18 +296,23 @@ class NativeEngine:
         if ent is not None:
             return ent
         dev = self.device
-        st = {'tokens': torch.zeros(B, dtype=torch.long, device=dev), 'positions': torch.zeros(B, dtype=torch.long, device=dev),
-              'table': torch.zeros(B, max_blocks, dtype=torch.int32, device=dev), 'seq_lens': torch.zeros(B, dtype=torch.int32, device=dev),
-              'slots': torch.zeros(B, dtype=torch.int32, device=dev)}
+        ints = torch.zeros(B * (max_blocks + 2), dtype=torch.int32, device=dev)       # filled by one copy per step
+        st = {'tokens': torch.zeros(B, dtype=torch.long, device=dev), 'ints': ints, 'table': ints[:B * max_blocks].view(B, max_blocks),
+              'seq_lens': ints[B * max_blocks:B * (max_blocks + 1)], 'slots': ints[B * (max_blocks + 1):]}
+
+        def body():
+            # the token of a step is the last of its sequence; rows that fill up the batch have length 0 and position 0
+            return self._decode_body(st['tokens'], (st['seq_lens'] - 1).clamp_min(0).long(), st['table'], st['seq_lens'], None, slots=st['slots'])
+
         side = torch.cuda.Stream(device=dev)
         side.wait_stream(torch.cuda.current_stream(dev))
         with torch.cuda.stream(side):  # warm-up outside the capture: one-time kernel attribute set-up, allocator warm-up
             for _ in range(2):
-                self._decode_body(st['tokens'], st['positions'], st['table'], st['seq_lens'], None, slots=st['slots'])
+                body()
         torch.cuda.current_stream(dev).wait_stream(side)
         graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(graph):
-            st['logits'] = self._decode_body(st['tokens'], st['positions'], st['table'], st['seq_lens'], None, slots=st['slots'])
+            st['logits'] = body()
         st['graph'] = graph
         self._graphs[key] = st
         return st
@@ -307,7 +323,6 @@ class NativeEngine:
         layer stack is a few dozen short kernels, so the step is replayed from a CUDA graph (one per batch-size
         bucket) unless adapters or routing capture need the eager path."""
         B = len(seqs)
-        positions = torch.tensor([s.length - 1 for s in seqs], device=self.device)
         max_blocks = max(len(s.blocks) for s in seqs)
         lora = self._lora_for(seqs, [1] * B)
         use_graph = (self.use_cuda_graphs and self.device.type == 'cuda' and lora is None and not self.capture_routing and not self.cfg.is_moe
@@ -325,22 +340,16 @@ class NativeEngine:
                 logging.getLogger('twinkle_b200').warning(f'CUDA-graph capture of the decode step failed ({type(e).__name__}: {e}); running eagerly')
                 st = None
             if st is not None:
-                table = torch.zeros(Bb, Mb, dtype=torch.int32)
-                for i, s in enumerate(seqs):
-                    table[i, :len(s.blocks)] = torch.tensor(s.blocks, dtype=torch.int32)
-                lens = torch.zeros(Bb, dtype=torch.int32)
-                lens[:B] = torch.tensor([s.length for s in seqs], dtype=torch.int32)
-                slots = torch.zeros(Bb, dtype=torch.int32)
-                slots[:B] = torch.tensor([s.state_slot for s in seqs], dtype=torch.int32)
-                st['slots'].copy_(slots, non_blocking=True)
-                st['table'].copy_(table, non_blocking=True)
-                st['seq_lens'].copy_(lens, non_blocking=True)
-                st['tokens'].zero_()
+                # a fresh pinned tensor each time: the allocator hands it out again only when the copy is done
+                ints = torch.empty(Bb * (Mb + 2), dtype=torch.int32, pin_memory=True)
+                ops.ext().pack_step(ints, Bb, Mb, [s.blocks for s in seqs], [s.length for s in seqs], [s.state_slot for s in seqs])
+                st['ints'].copy_(ints, non_blocking=True)
+                if B < Bb:
+                    st['tokens'].zero_()
                 st['tokens'][:B].copy_(last_tokens)
-                st['positions'].zero_()
-                st['positions'][:B].copy_(positions)
                 st['graph'].replay()
                 return st['logits'][:B]
+        positions = torch.tensor([s.length - 1 for s in seqs], device=self.device)
         table = torch.zeros(B, max_blocks, dtype=torch.int32, device=self.device)
         for i, s in enumerate(seqs):
             table[i, :len(s.blocks)] = torch.tensor(s.blocks, dtype=torch.int32)
