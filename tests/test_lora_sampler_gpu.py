@@ -495,3 +495,18 @@ def test_cache_write_places(E, dtype, hkv, d, e, lens):
     out = torch.full((4 * (5 + 2), ), -1, dtype=torch.int32)
     E.pack_step(out, 4, 5, [[7, 8, 9], [3]], [40, 2], [1, 2])
     assert out.tolist() == [7, 8, 9, 0, 0, 3, 0, 0, 0, 0] + [0] * 10 + [40, 2, 0, 0] + [1, 2, 0, 0]
+
+
+@pytest.mark.parametrize('H', [1024, 2048, 4096, 1032])
+@pytest.mark.parametrize('rows', [1, 2, 147, 297, 1500])
+def test_rmsnorm_rows_in_registers(E, H, rows):
+    """Widths with and without a kernel that keeps its rows, few rows and many, with a residual and without."""
+    x, r, w = torch.randn(rows, H, device='cuda').bfloat16(), torch.randn(rows, H, device='cuda').bfloat16(), torch.randn(H, device='cuda').bfloat16()
+    for res in (None, r):
+        got = E.rmsnorm_fwd(x, w, 1e-6, 0.5, res)
+        h = x if res is None else (x.float() + r.float()).bfloat16()
+        rstd = torch.rsqrt(h.double().pow(2).mean(-1) + 1e-6)
+        assert rel(got[1], rstd) < 4e-6                       # fp32 sums
+        assert rel(got[0], h.double() * rstd[:, None] * (w.double() + 0.5)) < 2.0 ** -8
+        if res is not None:
+            assert torch.equal(got[2], h)

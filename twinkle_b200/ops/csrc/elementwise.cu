@@ -68,6 +68,65 @@ __global__ void rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __res
   }
 }
 
+// The same for rows of NV·256 elements, which fit a warp's registers: every load of a row is on its way at once and the row is read once.
+// 64 x 4096 14.2 → 3.3 us (4.8 with a residual), 1 x 1024 4.4 → 2.1 (2.5): the latency of one load instead of two chains.
+template <int NV, bool RES>
+__global__ void rmsnorm_fwd_regs_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, const bf16* __restrict__ w, bf16* __restrict__ y, bf16* __restrict__ hsum,
+                                        float* __restrict__ rstd, int rows, float eps, float offset) {
+  constexpr int H = NV * 256;
+  const int warps_per_block = blockDim.x >> 5, lane = threadIdx.x & 31;
+  const uint4* wr = reinterpret_cast<const uint4*>(w);
+  for (int row = blockIdx.x * warps_per_block + (threadIdx.x >> 5); row < rows; row += gridDim.x * warps_per_block) {
+    const uint4* xr = reinterpret_cast<const uint4*>(x + static_cast<size_t>(row) * H);
+    uint4 u[NV];
+#pragma unroll
+    for (int i = 0; i < NV; ++i) u[i] = xr[i * 32 + lane];
+    float ss = 0.f;
+    if constexpr (RES) {
+      const uint4* rr = reinterpret_cast<const uint4*>(res + static_cast<size_t>(row) * H);
+      uint4* hr = reinterpret_cast<uint4*>(hsum + static_cast<size_t>(row) * H);
+      uint4 q[NV];
+#pragma unroll
+      for (int i = 0; i < NV; ++i) q[i] = rr[i * 32 + lane];
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        uint32_t* pu = &u[i].x;
+        const uint32_t* pq = &q[i].x;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2 a = unpack_bf16(pu[k]), b = unpack_bf16(pq[k]);
+          pu[k] = pack_bf16(a.x + b.x, a.y + b.y);
+          const float2 c = unpack_bf16(pu[k]);  // the norm sees the rounded sum, as it would after a separate add
+          ss += c.x * c.x + c.y * c.y;
+        }
+        hr[i * 32 + lane] = u[i];
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const float2 a = unpack_bf16(u[i].x), b = unpack_bf16(u[i].y), c = unpack_bf16(u[i].z), d = unpack_bf16(u[i].w);
+        ss += a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y + c.x * c.x + c.y * c.y + d.x * d.x + d.y * d.y;
+      }
+    }
+    ss = warp_sum(ss);
+    const float r = rsqrtf(ss / H + eps);
+    if (lane == 0) rstd[row] = r;
+    uint4* yr = reinterpret_cast<uint4*>(y + static_cast<size_t>(row) * H);
+#pragma unroll
+    for (int i = 0; i < NV; ++i) {
+      const uint4 ww = wr[i * 32 + lane];
+      const float2 a = unpack_bf16(u[i].x), b = unpack_bf16(u[i].y), c = unpack_bf16(u[i].z), d = unpack_bf16(u[i].w);
+      const float2 wa = unpack_bf16(ww.x), wb = unpack_bf16(ww.y), wc = unpack_bf16(ww.z), wd = unpack_bf16(ww.w);
+      uint4 o;
+      o.x = pack_bf16(a.x * r * (wa.x + offset), a.y * r * (wa.y + offset));
+      o.y = pack_bf16(b.x * r * (wb.x + offset), b.y * r * (wb.y + offset));
+      o.z = pack_bf16(c.x * r * (wc.x + offset), c.y * r * (wc.y + offset));
+      o.w = pack_bf16(d.x * r * (wd.x + offset), d.y * r * (wd.y + offset));
+      yr[i * 32 + lane] = o;
+    }
+  }
+}
+
 // dx = rstd·(g·w' − x·rstd²·mean(g·w'·x)),  dw += Σ_rows g·x·rstd.
 // Row-block form (H ≤ 8192): the whole block works on the same R rows at a time and a thread owns the same VPT 16-byte
 // column vectors in every row.  A row's g and x are read once into registers (2·R·VPT 16-byte loads per thread in
@@ -248,12 +307,24 @@ std::vector<torch::Tensor> rmsnorm_fwd(const torch::Tensor& x, const torch::Tens
   auto rstd = torch::empty({rows}, x.options().dtype(torch::kFloat32));
   torch::Tensor h = has_res ? torch::empty_like(x) : torch::Tensor();
   if (rows > 0) {
-    int blocks = std::min((rows + 7) / 8, num_sms() * 8);
-    rmsnorm_fwd_kernel<<<blocks, 256, 0, at::cuda::getCurrentCUDAStream()>>>(
-        reinterpret_cast<const bf16*>(x.data_ptr()), has_res ? reinterpret_cast<const bf16*>(residual->data_ptr()) : nullptr,
-        reinterpret_cast<const bf16*>(w.data_ptr()), reinterpret_cast<bf16*>(y.data_ptr()),
-        has_res ? reinterpret_cast<bf16*>(h.data_ptr()) : nullptr, rstd.data_ptr<float>(), rows, H, static_cast<float>(eps),
-        static_cast<float>(offset));
+    auto regs = [&](auto kern) {       // few rows are spread over the SMs
+      const int warps = std::max(1, std::min(8, rows / num_sms())), blocks = std::min((rows + warps - 1) / warps, num_sms() * 8);
+      kern<<<blocks, warps * 32, 0, at::cuda::getCurrentCUDAStream()>>>(
+          reinterpret_cast<const bf16*>(x.data_ptr()), has_res ? reinterpret_cast<const bf16*>(residual->data_ptr()) : nullptr, reinterpret_cast<const bf16*>(w.data_ptr()),
+          reinterpret_cast<bf16*>(y.data_ptr()), has_res ? reinterpret_cast<bf16*>(h.data_ptr()) : nullptr, rstd.data_ptr<float>(), rows, static_cast<float>(eps),
+          static_cast<float>(offset));
+    };
+    if (H == 1024) { if (has_res) regs(rmsnorm_fwd_regs_kernel<4, true>); else regs(rmsnorm_fwd_regs_kernel<4, false>); }
+    else if (H == 2048) { if (has_res) regs(rmsnorm_fwd_regs_kernel<8, true>); else regs(rmsnorm_fwd_regs_kernel<8, false>); }
+    else if (H == 4096) { if (has_res) regs(rmsnorm_fwd_regs_kernel<16, true>); else regs(rmsnorm_fwd_regs_kernel<16, false>); }
+    else {
+      int blocks = std::min((rows + 7) / 8, num_sms() * 8);
+      rmsnorm_fwd_kernel<<<blocks, 256, 0, at::cuda::getCurrentCUDAStream()>>>(
+          reinterpret_cast<const bf16*>(x.data_ptr()), has_res ? reinterpret_cast<const bf16*>(residual->data_ptr()) : nullptr,
+          reinterpret_cast<const bf16*>(w.data_ptr()), reinterpret_cast<bf16*>(y.data_ptr()),
+          has_res ? reinterpret_cast<bf16*>(h.data_ptr()) : nullptr, rstd.data_ptr<float>(), rows, H, static_cast<float>(eps),
+          static_cast<float>(offset));
+    }
     count_launch();
     TK_CUDA_CHECK(cudaGetLastError());
   }
@@ -365,7 +436,7 @@ __global__ void __launch_bounds__(256, 3) qk_norm_rope_fwd_kernel(const bf16* __
       }
     }
     const bf16* row = qkv + static_cast<size_t>(t) * heads * D + j * 8;
-    for (int h0 = 0; h0 < heads; h0 += 2 * ROPE_U) {
+    for (int h0 = blockIdx.y * 2 * ROPE_U; h0 < heads; h0 += gridDim.y * 2 * ROPE_U) {
       uint4 raw[ROPE_U];
 #pragma unroll
       for (int u = 0; u < ROPE_U; ++u) {
@@ -544,7 +615,9 @@ std::vector<torch::Tensor> qk_norm_rope_fwd(const torch::Tensor& qkv, const torc
   auto rstd = torch::empty({T, hq + hkv}, qkv.options().dtype(torch::kFloat32));
   if (T == 0) return {q, k, v, rstd};
   int blocks = static_cast<int>(std::max<long>(1, std::min<long>((T + 7L) / 8, num_sms() * 8L)));
-  qk_norm_rope_fwd_kernel<true><<<blocks, 256, 0, at::cuda::getCurrentCUDAStream()>>>(
+  // few tokens: their heads are shared out too (one token of 32 heads 7.6 → 3.6 us, 64 of 48 11.8 → 4.3)
+  const int chunks = blocks < num_sms() ? static_cast<int>((hq + 2 * hkv + 2 * ROPE_U - 1) / (2 * ROPE_U)) : 1;
+  qk_norm_rope_fwd_kernel<true><<<dim3(blocks, chunks), 256, 0, at::cuda::getCurrentCUDAStream()>>>(
       reinterpret_cast<const bf16*>(qkv.data_ptr()), reinterpret_cast<const bf16*>(qw.data_ptr()), reinterpret_cast<const bf16*>(kw.data_ptr()),
       cosb.data_ptr<float>(), sinb.data_ptr<float>(), reinterpret_cast<bf16*>(q.data_ptr()), reinterpret_cast<bf16*>(k.data_ptr()),
       reinterpret_cast<bf16*>(v.data_ptr()), rstd.data_ptr<float>(), T, hq, hkv, static_cast<float>(eps));
