@@ -206,13 +206,16 @@ static void launch_paged_decode(const torch::Tensor& q, const torch::Tensor& kc,
         reinterpret_cast<const T*>(vc.data_ptr()), tables.data_ptr<int>(), seq_lens.data_ptr<int>(), reinterpret_cast<T*>(out.data_ptr()), hq, hkv, d, e,
         static_cast<int>(kc.size(1)), static_cast<int>(tables.size(1)), sl2, G, extras);
   };
+  // Where the CTAs leave SMs idle a head has one of its own: a step is bound by the instructions of a warp per token, not by the rows that two CTAs
+  // then read (one sequence of 1 k tokens, 16/8 heads of 128: 20.6 → 19.3 us), and every head is computed as before.
+  const bool alone = static_cast<long>(B) * hq <= 2 * num_sms();
   const int vectors = (std::max(d, e) + 8 * V - 1) / (8 * V);   // per lane
   if (vectors <= 1) {
-    if (G == 1) go(paged_decode_kernel<T, 1, 1, 2, TERMS>, 1); else if (G == 2) go(paged_decode_kernel<T, 2, 1, 2, TERMS>, 2); else go(paged_decode_kernel<T, 4, 1, 2, TERMS>, 4);
+    if (G == 1 || alone) go(paged_decode_kernel<T, 1, 1, 2, TERMS>, 1); else if (G == 2) go(paged_decode_kernel<T, 2, 1, 2, TERMS>, 2); else go(paged_decode_kernel<T, 4, 1, 2, TERMS>, 4);
   } else if (vectors <= 2) {
-    if (G == 1) go(paged_decode_kernel<T, 1, 2, 2, TERMS>, 1); else if (G == 2) go(paged_decode_kernel<T, 2, 2, 2, TERMS>, 2); else go(paged_decode_kernel<T, 4, 2, 2, TERMS>, 4);
+    if (G == 1 || alone) go(paged_decode_kernel<T, 1, 2, 2, TERMS>, 1); else if (G == 2) go(paged_decode_kernel<T, 2, 2, 2, TERMS>, 2); else go(paged_decode_kernel<T, 4, 2, 2, TERMS>, 4);
   } else if (vectors <= 4) {
-    if (G == 1) go(paged_decode_kernel<T, 1, 4, 1, TERMS>, 1); else go(paged_decode_kernel<T, 2, 4, 1, TERMS>, 2);
+    if (G == 1 || alone) go(paged_decode_kernel<T, 1, 4, 1, TERMS>, 1); else go(paged_decode_kernel<T, 2, 4, 1, TERMS>, 2);
   } else if constexpr (sizeof(T) == 4) {   // 16-bit rows of up to 256 elements are four vectors per lane
     go(paged_decode_kernel<T, 1, 8, 1, TERMS>, 1);
   }
