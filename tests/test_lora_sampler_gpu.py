@@ -510,3 +510,43 @@ def test_rmsnorm_rows_in_registers(E, H, rows):
         assert rel(got[0], h.double() * rstd[:, None] * (w.double() + 0.5)) < 2.0 ** -8
         if res is not None:
             assert torch.equal(got[2], h)
+
+
+@pytest.mark.parametrize('lens,klens', [((130, 300), (0, 40)), ((5, 400), (5, 100)), ((0, 200, 3), (300, 200, 0)), ((260, 129), (30, 0))])
+@pytest.mark.parametrize('causal', [True, False])
+@pytest.mark.parametrize('hq,hkv', [(8, 1), (64, 32)])
+def test_flash_tiles_without_keys(E, lens, klens, causal, hq, hkv):
+    """Query tiles that see no key and key tiles that no query sees: zeros, and −inf for the log-sum-exp, as for such rows of other tiles."""
+    from twinkle_b200 import ops
+    g = torch.Generator(device='cuda').manual_seed(sum(lens))
+    q, k, v, do = (torch.randn(n, h, 128, device='cuda', generator=g).bfloat16() for n, h in ((sum(lens), hq), (sum(klens), hkv), (sum(klens), hkv), (sum(lens), hq)))
+    cu, cuk = (torch.tensor([0] + list(x), device='cuda').cumsum(0).int() for x in (lens, klens))
+    leaves = [t.clone().requires_grad_() for t in (q, k, v)]
+    o, lse = ops.flash_attn_varlen(*leaves, cu, max(lens), causal=causal, cu_seqlens_k=cuk, max_seqlen_k=max(klens), return_lse=True)
+    got = torch.autograd.grad(o, leaves, do)
+    ref = [t.double().requires_grad_() for t in (q, k, v)]
+    want, dead, a, b = torch.zeros_like(ref[0]), torch.ones(sum(lens), dtype=torch.bool, device='cuda'), 0, 0
+    for n, m in zip(lens, klens):
+        first = max(0, n - m) if causal else 0                # rows before it see nothing
+        if m and first < n:
+            kk, vv = (t[b:b + m].repeat_interleave(hq // hkv, 1) for t in ref[1:])
+            s = torch.einsum('qhd,khd->hqk', ref[0][a + first:a + n], kk) * 128 ** -0.5
+            if causal:
+                s = s.masked_fill(torch.ones(n - first, m, dtype=torch.bool, device='cuda').triu(m - n + first + 1), float('-inf'))
+            want = want.index_add(0, torch.arange(a + first, a + n, device='cuda'), torch.einsum('hqk,khd->qhd', torch.softmax(s, -1), vv))
+            dead[a + first:a + n] = False
+        a, b = a + n, b + m
+    assert not o[dead].any() and (lse[:, dead] == float('-inf')).all() and lse[:, ~dead].isfinite().all()
+    assert not got[0][dead].any()
+    for x, y in zip((o, *got), (want, *torch.autograd.grad(want, ref, do.double()))):
+        assert rel(x, y) < 8e-3        # P and dS rounded to bf16 (2^-9 each at most) and the result too
+    # keys of three chunks: one query tile per CTA
+    q, k, v = (torch.randn(n, h, w, device='cuda', generator=g).bfloat16() for n, h, w in ((sum(lens), hq, 192), (sum(klens), hkv, 192), (sum(klens), hkv, 64)))
+    o, lse = E.flash_attn_fwd(q, k, v, cu, max(lens), causal, 192 ** -0.5, cuk)
+    assert not o[dead].any() and (lse[:, dead] == float('-inf')).all() and o.isfinite().all() and o[~dead].any()
+    sinks = torch.randn(hq, device='cuda', generator=g).bfloat16()
+    for w in (128, 192):
+        q, k, v = (torch.randn(n, h, w, device='cuda', generator=g).bfloat16() for n, h in ((sum(lens), hq), (sum(klens), hkv), (sum(klens), hkv)))
+        o, lse = E.flash_attn_fwd(q, k, v[..., :128].contiguous(), cu, max(lens), causal, w ** -0.5, cuk, sinks)
+        assert not o[dead].any() and torch.equal(lse[:, dead], sinks.float()[:, None].expand(-1, int(dead.sum())))
+    assert E.read_and_clear_error() == 0

@@ -136,7 +136,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
   if (warp == 8) {
     // producer warp: lane 0 drives TMA; all lanes stage lse (log2 units) and δ of each query block in smem
-    if (lane == 0) {
+    if (lane == 0 && n_iter > 0) {     // a tile that no query sees loads nothing: nobody would wait for it
       mbar_expect_tx(kv_full, 2 * TILE_BYTES);
       tma_load_3d(smem + SMEM_A, &tmK, kv_full, 0, kv_head, kv_start + kv0);
       tma_load_3d(smem + SMEM_A + ATOM, &tmK, kv_full, 64, kv_head, kv_start + kv0);
@@ -222,7 +222,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       add_up(t_dk, t_dp, SMEM_X + st * TILE_BYTES, it == 0, &qdo_empty[st]);    // dK += dSᵀ·Q
       if (more) scores(t_dp, dV, SMEM_Y + nx * TILE_BYTES, dp_full);
     }
-    if (elect_one()) umma_commit(acc_done);
+    if (n_iter > 0 && elect_one()) umma_commit(acc_done);
     __syncwarp();
   }
   bool ok = true;
@@ -336,7 +336,7 @@ flash_bwd_dkdv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         }
       }
     } else if (n_iter == 0 && row_valid && rank == 0) {
-      // no query attends to this tile (cannot happen with causal self-attention, kept for safety)
+      // no query sees this tile (keys of a sequence without queries, or all of them behind every query)
       for (int i = wg * 64; i < wg * 64 + 64; i += 8) {
         *reinterpret_cast<uint4*>(dkrow + i) = make_uint4(0, 0, 0, 0);
         *reinterpret_cast<uint4*>(dvrow + i) = make_uint4(0, 0, 0, 0);
@@ -423,7 +423,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t t_dp = tmem_base + 256, t_dq = tmem_base + 384;
 
   if (warp == 8) {
-    if (lane == 0) {
+    if (lane == 0 && n_iter > 0) {
       mbar_expect_tx(qdo_full, 2 * TILE_BYTES);
       tma_load_3d(smem + SMEM_A, &tmQ, qdo_full, 0, head, seq_start + q0);
       tma_load_3d(smem + SMEM_A + ATOM, &tmQ, qdo_full, 64, head, seq_start + q0);
@@ -482,7 +482,7 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       }
       __syncwarp();
     }
-    if (elect_one()) umma_commit(acc_done);
+    if (n_iter > 0 && elect_one()) umma_commit(acc_done);
     __syncwarp();
   } else {
     const int wg = warp >> 2;
@@ -534,9 +534,9 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       tc_fence_before();
       mbar_arrive(&ds_ready[it & 1]);
     }
+    bf16* dqrow = p.dq + (static_cast<size_t>(seq_start + q_pos) * p.hq + head) * D;
     if (ok && n_iter > 0 && mbar_wait(acc_done, 0, p.err, ERR_ATTN_WAIT)) {
       tc_fence_after();
-      bf16* dqrow = p.dq + (static_cast<size_t>(seq_start + q_pos) * p.hq + head) * D;
 #pragma unroll 1
       for (int c = 2 * wg; c < 2 * wg + 2; ++c) {
         uint32_t a[32];
@@ -552,6 +552,8 @@ flash_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
                            pack_bf16(__uint_as_float(a[i + 6]) * p.scale, __uint_as_float(a[i + 7]) * p.scale));
         }
       }
+    } else if (n_iter == 0 && row_valid) {          // queries before all keys
+      for (int i = wg * 64; i < wg * 64 + 64; i += 8) *reinterpret_cast<uint4*>(dqrow + i) = make_uint4(0u, 0u, 0u, 0u);
     }
   }
   tc_fence_before();

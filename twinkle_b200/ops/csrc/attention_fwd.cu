@@ -105,6 +105,14 @@ __device__ __forceinline__ void store_out(const FwdParams& p, uint32_t tmem_row,
   }
 }
 
+// A row that sees no key: nothing comes out, and its log-sum-exp is the sink's logit or −∞.
+__device__ __forceinline__ float empty_lse(const FwdParams& p, int head) { return p.sinks != nullptr ? __bfloat162float(p.sinks[head]) : -INFINITY; }
+__device__ __forceinline__ void store_empty(const FwdParams& p, int head, int token) {
+  bf16* orow = p.out + (static_cast<size_t>(token) * p.hq + head) * p.e;
+  for (int i = 0; i < p.e; i += 8) *reinterpret_cast<uint4*>(orow + i) = make_uint4(0u, 0u, 0u, 0u);
+  p.lse[static_cast<size_t>(head) * p.T + token] = empty_lse(p, head);
+}
+
 // KA / VA: 64-wide chunks of a query / key row (up to 3) and of a value row (1 or 2).
 template <int KA, int VA, bool TERMS>
 __global__ void __launch_bounds__(fa::THREADS, 1)
@@ -169,7 +177,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
 
   if (warp == 8) {
     // ------------------------------------------------------------- producer
-    if (lane == 0) {
+    if (lane == 0 && n_blocks > 0) {       // nobody would wait for the query
       tma_prefetch_desc(&tmQ);
       tma_prefetch_desc(&tmK);
       tma_prefetch_desc(&tmV);
@@ -216,7 +224,7 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       }
       __syncwarp();
     };
-    bool ok = wait(q_full, 0) && wait(&k_full[0], 0);
+    bool ok = n_blocks > 0 && wait(q_full, 0) && wait(&k_full[0], 0);
     if (ok) {
       tc_fence_after();
       issue_s(0);
@@ -379,7 +387,9 @@ flash_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (p.sinks != nullptr) l_sum += exp2f(__bfloat162float(p.sinks[head]) * 1.4426950408889634f - m_used);
       const bool valid = q_pos < seq_len;
       store_out<VA>(p, tmem_o + lane_off, head, seq_start + q_pos, valid, (l_sum > 0.f) ? 1.f / l_sum : 0.f, 2 * wg, 2 * wg + 2);
-      if (valid && wg == 0) p.lse[static_cast<size_t>(head) * p.T + seq_start + q_pos] = (m_used + log2f(l_sum)) * 0.6931471805599453f;
+      if (valid && wg == 0) p.lse[static_cast<size_t>(head) * p.T + seq_start + q_pos] = m_used == -INFINITY ? empty_lse(p, head) : (m_used + log2f(l_sum)) * 0.6931471805599453f;
+    } else if (n_blocks == 0 && wg == 0 && q_pos < seq_len) {
+      store_empty(p, head, seq_start + q_pos);
     }
   }
   tc_fence_before();
@@ -626,7 +636,9 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       if (p.sinks != nullptr) l_sum += exp2f(__bfloat162float(p.sinks[head]) * 1.4426950408889634f - m_used);
       const bool valid = q_pos < seq_len;
       store_out<VA>(p, to, head, seq_start + q_pos, valid, (l_sum > 0.f) ? 1.f / l_sum : 0.f, 0, 2 * VA);
-      if (valid) p.lse[static_cast<size_t>(head) * p.T + seq_start + q_pos] = (m_used + log2f(l_sum)) * 0.6931471805599453f;
+      if (valid) p.lse[static_cast<size_t>(head) * p.T + seq_start + q_pos] = m_used == -INFINITY ? empty_lse(p, head) : (m_used + log2f(l_sum)) * 0.6931471805599453f;
+    } else if (n_blocks == 0 && q_pos < seq_len) {
+      store_empty(p, head, seq_start + q_pos);
     }
   }
   tc_fence_before();
