@@ -1,0 +1,46 @@
+"""Parts of the CUDA sources that are plain C++, compiled and run on the host."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), 'twinkle_b200', 'ops', 'csrc')
+pytestmark = pytest.mark.skipif(shutil.which('g++') is None, reason='needs g++')
+
+
+def run_cpp(tmp_path, source):
+    (tmp_path / 'unit.cpp').write_text(source)
+    subprocess.run(['g++', '-std=c++17', '-O1', '-Wall', '-Werror', '-pthread', '-I', CSRC, 'unit.cpp', '-o', 'unit'], cwd=tmp_path, check=True, capture_output=True, text=True, timeout=120)
+    return subprocess.run(['./unit'], cwd=tmp_path, check=True, capture_output=True, text=True, timeout=60).stdout
+
+
+def test_a_producer_that_gives_up_waits_for_every_fill_under_way_and_for_no_other(tmp_path):
+    """Barriers as hardware has them: a wait on a parity passes unless the phase in progress has it.  For every number of fills issued and landed (in
+    order), the waits of the give-up path pass exactly when the last fill of each stage has landed."""
+    out = run_cpp(tmp_path, r'''
+#include <cstdio>
+#include <vector>
+#include "ring.h"
+int main() {
+  int bad = 0, checked = 0;
+  for (int stages = 1; stages <= 5; ++stages)
+    for (int issued = 0; issued <= 4 * stages; ++issued)
+      for (int landed = tk::ring_first_open(issued, stages); landed <= issued; ++landed) {
+        std::vector<int> phases(stages, 0);              // completed phases of each stage's barrier
+        for (int i = 0; i < landed; ++i) ++phases[i % stages];
+        bool done = true;
+        for (int i = tk::ring_first_open(issued, stages); i < issued; ++i) {
+          const tk::RingFill f = tk::ring_fill(i, stages);
+          const bool passes = (phases[f.stage] & 1u) != f.parity;
+          if (passes != (i < landed)) ++bad;
+          done = done && passes;
+        }
+        if (done != (landed == issued)) ++bad;
+        ++checked;
+      }
+  std::printf("%d %d", bad, checked);
+}
+''')
+    bad, checked = map(int, out.split())
+    assert bad == 0 and checked > 100

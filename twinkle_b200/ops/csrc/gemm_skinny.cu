@@ -18,6 +18,7 @@
 #include "common.cuh"
 #include "elect.cuh"
 #include "host.h"
+#include "ring.h"
 
 namespace tk {
 
@@ -81,7 +82,10 @@ __global__ void __launch_bounds__(gs::THREADS) gemm_skinny_kernel(const __grid_c
       int st = 0, ph = 0;
       for (int s = s0; s < s1; ++s) {
         if (!mbar_wait(&empty[st], ph ^ 1, p.err, ERR_PRODUCER_WAIT)) {
-          for (int i = 0; i < p.stages; ++i) mbar_wait(&full[i], 0, nullptr, 0);     // copies in flight land, within the limit, before the CTA exits
+          for (int i = ring_first_open(s - s0, p.stages); i < s - s0; ++i) {     // copies in flight land, within the limit, before the CTA exits
+            const RingFill f = ring_fill(i, p.stages);
+            mbar_wait(&full[f.stage], f.parity, nullptr, 0);
+          }
           break;
         }
         mbar_expect_tx(&full[st], stage_bytes);     // atoms past K and rows past the tensors arrive as zeros
