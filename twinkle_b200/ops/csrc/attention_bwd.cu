@@ -591,13 +591,12 @@ std::vector<torch::Tensor> flash_attn_bwd(const torch::Tensor& dout, const torch
     TORCH_CHECK(cu_k->is_cuda() && cu_k->scalar_type() == torch::kInt32 && cu_k->is_contiguous() && cu_k->numel() == cu.numel(), "cu_k like cu");
     p.cu_k = cu_k->data_ptr<int>();
   }
-  static bool configured = false;
-  if (!configured) {
+  static OncePerDevice limit;
+  limit(current_device(), [] {
     TK_CUDA_CHECK(cudaFuncSetAttribute(flash_bwd_dkdv_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, fb::SMEM_TOTAL));
     TK_CUDA_CHECK(cudaFuncSetAttribute(flash_bwd_dkdv_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, fb::SMEM_TOTAL));
     TK_CUDA_CHECK(cudaFuncSetAttribute(flash_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fb::SMEM_TOTAL));
-    configured = true;
-  }
+  });
   const int tiles = (static_cast<int>(max_seqlen) + fb::BT - 1) / fb::BT;
   const int tiles_k = (static_cast<int>(max_seqlen_k > 0 ? max_seqlen_k : max_seqlen) + fb::BT - 1) / fb::BT;
   CUtensorMap tq = make_head_tmap(q, fb::BT), tdo = make_head_tmap(dout, fb::BT), tk_ = make_head_tmap(k, fb::BT), tv = make_head_tmap(v, fb::BT);

@@ -702,11 +702,8 @@ std::vector<torch::Tensor> flash_attn_fwd(const torch::Tensor& q, const torch::T
   auto stream = at::cuda::getCurrentCUDAStream();
 #define TK_FLASH_RUN(KA, VA, TERMS)                                                                                                     \
   do {                                                                                                                                  \
-    static bool configured = false;                                                                                                     \
-    if (!configured) {                                                                                                                  \
-      TK_CUDA_CHECK(cudaFuncSetAttribute(flash_fwd_kernel<KA, VA, TERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, fa::Smem<KA>::TOTAL));  \
-      configured = true;                                                                                                                \
-    }                                                                                                                                   \
+    static OncePerDevice limit;                                                                                                         \
+    limit(current_device(), [] { TK_CUDA_CHECK(cudaFuncSetAttribute(flash_fwd_kernel<KA, VA, TERMS>, cudaFuncAttributeMaxDynamicSharedMemorySize, fa::Smem<KA>::TOTAL)); });\
     flash_fwd_kernel<KA, VA, TERMS><<<grid, fa::THREADS, fa::Smem<KA>::TOTAL, stream>>>(tq, tk_, tv, tr, p);                                   \
   } while (0)
   const bool wide_k = chunks > 1, wide_v = v.size(2) > 64;
@@ -714,18 +711,15 @@ std::vector<torch::Tensor> flash_attn_fwd(const torch::Tensor& q, const torch::T
   const bool pairs = chunks <= 2 && !p.terms.used;
   if (pairs) {
     const dim3 half(hq, (grid.y + 1) / 2, nseq);
-    auto go = [&](auto kern, bool& configured) {
-      if (!configured) {
-        TK_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fa2::TOTAL));
-        configured = true;
-      }
+    auto go = [&](auto kern, OncePerDevice& limit) {
+      limit(current_device(), [=] { TK_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, fa2::TOTAL)); });
       kern<<<half, fa::THREADS, fa2::TOTAL, stream>>>(tq, tk_, tv, tr, p);
     };
-    static bool configured[4];
-    if (wide_k && wide_v) go(flash_fwd_pair_kernel<2, 2>, configured[0]);
-    else if (wide_k) go(flash_fwd_pair_kernel<2, 1>, configured[1]);
-    else if (wide_v) go(flash_fwd_pair_kernel<1, 2>, configured[2]);
-    else go(flash_fwd_pair_kernel<1, 1>, configured[3]);
+    static OncePerDevice limits[4];
+    if (wide_k && wide_v) go(flash_fwd_pair_kernel<2, 2>, limits[0]);
+    else if (wide_k) go(flash_fwd_pair_kernel<2, 1>, limits[1]);
+    else if (wide_v) go(flash_fwd_pair_kernel<1, 2>, limits[2]);
+    else go(flash_fwd_pair_kernel<1, 1>, limits[3]);
     count_launch();
     TK_CUDA_CHECK(cudaGetLastError());
     return {out, lse};

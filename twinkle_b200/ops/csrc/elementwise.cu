@@ -368,11 +368,8 @@ std::vector<torch::Tensor> rmsnorm_bwd(const torch::Tensor& g, const torch::Tens
   while (warps > 1 && static_cast<size_t>(warps) * H * sizeof(float) > 200 * 1024) warps >>= 1;
   const size_t smem = static_cast<size_t>(warps) * H * sizeof(float);
   TORCH_CHECK(smem <= 200 * 1024, "hidden size too large for the RMSNorm backward kernel");
-  static size_t configured = 0;
-  if (smem > 48 * 1024 && smem > configured) {
-    TK_CUDA_CHECK(cudaFuncSetAttribute(rmsnorm_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    configured = 200 * 1024;
-  }
+  static OncePerDevice limit;
+  limit(current_device(), [] { TK_CUDA_CHECK(cudaFuncSetAttribute(rmsnorm_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); });
   int blocks = std::min((rows + warps - 1) / warps, num_sms());
   rmsnorm_bwd_kernel<<<blocks, warps * 32, smem, at::cuda::getCurrentCUDAStream()>>>(
       reinterpret_cast<const bf16*>(g.data_ptr()), reinterpret_cast<const bf16*>(x.data_ptr()), reinterpret_cast<const bf16*>(w.data_ptr()),

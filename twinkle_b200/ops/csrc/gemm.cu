@@ -362,12 +362,9 @@ static void launch(bool a_mn, bool b_mn, int mode, const CUtensorMap& ta, const 
   if (grid <= 0) return;
 #define TK_LAUNCH(AM, BMN, MD)                                                                                   \
   do {                                                                                                           \
-    static bool configured = false;                                                                              \
+    static OncePerDevice limit;                                                                                  \
     auto kern = gemm_tcgen05_kernel<AM, BMN, MD>;                                                                \
-    if (!configured) {                                                                                           \
-      TK_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));        \
-      configured = true;                                                                                         \
-    }                                                                                                            \
+    limit(current_device(), [=] { TK_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES)); });\
     kern<<<grid, GEMM_THREADS, SMEM_BYTES, stream>>>(ta, tb, xa2, xb2, p);                                        \
   } while (0)
   if (mode == 0) {

@@ -26,6 +26,8 @@
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/types.h>
 
+#include <atomic>
+
 #include "common.cuh"
 #include "host.h"
 
@@ -501,26 +503,28 @@ bool gemm_pair_launch(bool a_mn, bool b_mn, const CUtensorMap& ta, const CUtenso
   const int tiles = ((M + g2::TM - 1) / g2::TM) * ((N + g2::TN - 1) / g2::TN);
 #define TK_LAUNCH2(AM, BMN)                                                                                            \
   do {                                                                                                                 \
-    static int pairs = -1;                                                                                             \
-    auto kern = g2::gemm_tcgen05_pair_kernel<AM, BMN, g2::FUSE_NONE>;                                                                 \
-    if (pairs < 0) {                                                                                                   \
+    static OncePerDevice limit;                                                                                        \
+    static std::atomic<int> pairs{-1};                                                                                 \
+    auto kern = g2::gemm_tcgen05_pair_kernel<AM, BMN, g2::FUSE_NONE>;                                                  \
+    limit(current_device(), [=] {                                                                                      \
       TK_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, g2::SMEM_BYTES));          \
       pairs = max_pairs(kern);                                                                                         \
-    }                                                                                                                  \
+    });                                                                                                                \
     if (pairs <= 0) return false;                                                                                      \
-    const int grid = 2 * std::min(tiles, std::min(pairs, num_sms() / 2));                                              \
+    const int grid = 2 * std::min(tiles, std::min(pairs.load(), num_sms() / 2));                                              \
     kern<<<grid, g2::THREADS, g2::SMEM_BYTES, stream>>>(ta, tb, ta, p);                                                \
   } while (0)
 #define TK_LAUNCH2S(AM, BMN)                                                                                           \
   do {                                                                                                                 \
-    static int pairs = -1;                                                                                             \
+    static OncePerDevice limit;                                                                                        \
+    static std::atomic<int> pairs{-1};                                                                                 \
     auto kern = g2::gemm_tcgen05_pair_kernel<AM, BMN, g2::FUSE_STAGED>;                                                \
-    if (pairs < 0) {                                                                                                   \
+    limit(current_device(), [=] {                                                                                      \
       TK_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, g2::SMEM_BYTES));          \
       pairs = max_pairs(kern);                                                                                         \
-    }                                                                                                                  \
+    });                                                                                                                \
     if (pairs <= 0) return false;                                                                                      \
-    const int grid = 2 * std::min(tiles, std::min(pairs, num_sms() / 2));                                              \
+    const int grid = 2 * std::min(tiles, std::min(pairs.load(), num_sms() / 2));                                              \
     kern<<<grid, g2::THREADS, g2::SMEM_BYTES, stream>>>(ta, tb, ta, p);                                                \
   } while (0)
   const bool staged = g_staged_epilogue && !out_fp32 && !accumulate && N % 8 == 0;
@@ -555,14 +559,15 @@ static void launch_fused(bool b_mn, const CUtensorMap& ta, const CUtensorMap& tb
   const int tiles = ((p.M + g2::TM - 1) / g2::TM) * ((p.N + g2::TN - 1) / g2::TN);
 #define TK_LAUNCH_F(BMN)                                                                                               \
   do {                                                                                                                 \
-    static int pairs = -1;                                                                                             \
+    static OncePerDevice limit;                                                                                        \
+    static std::atomic<int> pairs{-1};                                                                                 \
     auto kern = g2::gemm_tcgen05_pair_kernel<false, BMN, FUSE>;                                                        \
-    if (pairs < 0) {                                                                                                   \
+    limit(current_device(), [=] {                                                                                      \
       TK_CUDA_CHECK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, g2::SMEM_BYTES));          \
       pairs = max_pairs(kern);                                                                                         \
-    }                                                                                                                  \
+    });                                                                                                                \
     TORCH_CHECK(pairs > copy_ctas / 2, "SM-pair kernel cannot be resident on this device");                           \
-    const int avail = std::min(pairs, num_sms() / 2) - copy_ctas / 2;                                                  \
+    const int avail = std::min(pairs.load(), num_sms() / 2) - copy_ctas / 2;                                                  \
     const int grid = copy_ctas + 2 * std::min(tiles, avail);                                                           \
     kern<<<grid, g2::THREADS, g2::SMEM_BYTES, stream>>>(ta, tb, tl, p);                                                \
   } while (0)

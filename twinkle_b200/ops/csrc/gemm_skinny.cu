@@ -239,11 +239,10 @@ bool gemm_skinny(const torch::Tensor& a, const torch::Tensor& b, void* out, int 
   CUtensorMap ta = make_tmap_3d(a.data_ptr(), ATOM, M, p.k_atoms, a.stride(0), ATOM, ATOM, p.rows, ka);
   CUtensorMap tb = make_tmap_3d(b.data_ptr(), ATOM, N, p.k_atoms, b.stride(0), ATOM, ATOM, p.bn, ka);
   auto kern = ka == 4 ? gemm_skinny_kernel<4> : ka == 2 ? gemm_skinny_kernel<2> : gemm_skinny_kernel<1>;
-  static bool configured = false;
-  if (!configured) {
+  static OncePerDevice limit;
+  limit(current_device(), [] {
     for (auto k : {gemm_skinny_kernel<4>, gemm_skinny_kernel<2>, gemm_skinny_kernel<1>}) TK_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, 226 * 1024));
-    configured = true;
-  }
+  });
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(tiles * p.split, mt);
   cfg.blockDim = dim3(THREADS);

@@ -14,10 +14,15 @@ static std::atomic<long> g_launches{0};
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 long launch_count() { return g_launches.load(std::memory_order_relaxed); }
 
-int num_sms() {
-  static std::vector<int> cache(64, 0);
+int current_device() {
   int dev = 0;
   TK_CUDA_CHECK(cudaGetDevice(&dev));
+  return dev;
+}
+
+int num_sms() {
+  static std::vector<int> cache(64, 0);
+  const int dev = current_device();
   if (cache[dev] == 0) {
     cudaDeviceProp prop;
     TK_CUDA_CHECK(cudaGetDeviceProperties(&prop, dev));

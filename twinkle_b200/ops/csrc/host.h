@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <torch/types.h>
 
+#include "once_per_device.h"
+
 #define TK_CUDA_CHECK(expr)                                                                              \
   do {                                                                                                   \
     cudaError_t _e = (expr);                                                                             \
@@ -15,6 +17,9 @@ namespace tk {
 // Launch counter: every kernel launch issued by this extension bumps it (read by benchmarks).
 void count_launch(int n = 1);
 long launch_count();
+
+// The current device.
+int current_device();
 
 // Number of SMs of the current device (cached).
 int num_sms();

@@ -226,11 +226,8 @@ static int cluster_size(const PagedDecode& p, int B, int groups) {
 
 template <int D>
 static void launch(const PagedDecode& p, int B, cudaStream_t stream) {
-  static bool configured = false;
-  if (!configured) {
-    TK_CUDA_CHECK(cudaFuncSetAttribute(paged_decode_mma_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, pd::smem_bytes<D>()));
-    configured = true;
-  }
+  static OncePerDevice limit;
+  limit(current_device(), [] { TK_CUDA_CHECK(cudaFuncSetAttribute(paged_decode_mma_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, pd::smem_bytes<D>())); });
   const int groups = (p.G + pd::HEADS - 1) / pd::HEADS, S = cluster_size(p, B, groups);
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(S, p.hkv * groups, B);

@@ -369,11 +369,8 @@ std::vector<torch::Tensor> sample_tokens(const torch::Tensor& logits, double tem
   attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
   cfg.attrs = &attr;
   cfg.numAttrs = 1;
-  static bool configured = false;
-  if (!configured) {
-    TK_CUDA_CHECK(cudaFuncSetAttribute(sample_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRoom * 4));
-    configured = true;
-  }
+  static OncePerDevice limit;
+  limit(current_device(), [] { TK_CUDA_CHECK(cudaFuncSetAttribute(sample_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kRoom * 4)); });
   TK_CUDA_CHECK(cudaLaunchKernelEx(&cfg, cached ? sample_kernel<true> : sample_kernel<false>, static_cast<const float*>(logits.data_ptr<float>()),
                                    static_cast<const int64_t*>(seeds.data_ptr<int64_t>()), tok.data_ptr<int64_t>(), lp.data_ptr<float>(), V, part,
                                    greedy ? 1.f : static_cast<float>(1.0 / temperature), static_cast<int>(top_k), static_cast<float>(top_p), greedy ? 1 : 0, list_cap));
