@@ -550,3 +550,30 @@ def test_flash_tiles_without_keys(E, lens, klens, causal, hq, hkv):
         o, lse = E.flash_attn_fwd(q, k, v[..., :128].contiguous(), cu, max(lens), causal, w ** -0.5, cuk, sinks)
         assert not o[dead].any() and torch.equal(lse[:, dead], sinks.float()[:, None].expand(-1, int(dead.sum())))
     assert E.read_and_clear_error() == 0
+
+
+def test_cache_rows_outside_the_pool_are_an_error(E):
+    """Rows outside the pools are not written, the others are, and generation raises instead of going on without those keys."""
+    from twinkle_b200 import ops
+    from twinkle_b200.data_format import SamplingParams
+    from twinkle_b200.models import build_model
+    from twinkle_b200.sampler.engine import NativeEngine
+    assert E.read_and_clear_error() == 0
+    k, v = (torch.randn(4, 2, 64, device='cuda').bfloat16() for _ in range(2))
+    for bad in (-1, 48, 2**40):
+        kp, vp = (torch.zeros(3, 16, 2, 64, device='cuda', dtype=torch.bfloat16) for _ in range(2))
+        ops.cache_write(kp, vp, torch.tensor([5, bad, 0, 47], device='cuda'), k, v)
+        assert E.read_and_clear_error() == 7
+        for p, x in ((kp, k), (vp, v)):
+            want = torch.zeros_like(p).view(48, 2, 64)
+            want[[5, 0, 47]] = x[[0, 2, 3]]
+            assert torch.equal(p.view(48, 2, 64), want)
+    cfg = _tiny()
+    eng = NativeEngine(build_model(cfg, device='cuda', dtype=torch.bfloat16, seed=0), cfg, num_blocks=64, block_size=16)
+    places = eng._prompt_rows
+    eng._prompt_rows = lambda seqs, lens: places(seqs, lens) + 64 * 16
+    with pytest.raises(RuntimeError, match='error 7'):
+        eng.generate([[1, 2, 3]], [SamplingParams(max_tokens=2, temperature=0.0)])
+    eng._prompt_rows = places
+    assert len(eng.generate([[1, 2, 3]], [SamplingParams(max_tokens=2, temperature=0.0)])[0].sequences[0].tokens) == 2
+    assert E.read_and_clear_error() == 0

@@ -817,7 +817,8 @@ def paged_attention_decode(q, k_cache, v_cache, block_tables, seq_lens, scale: O
 
 
 def cache_write(k_pool, v_pool, rows, k, v) -> None:
-    """Store ``k, v [T, heads, width]`` in rows ``rows [T]`` (block · block size + offset) of the paged pools ``[blocks, block size, heads, width]``."""
+    """Store ``k, v [T, heads, width]`` in rows ``rows [T]`` (block · block size + offset) of the paged pools ``[blocks, block size, heads, width]``.
+    The kernel leaves out a row outside the pools and sets the error word, which ``NativeEngine.generate`` raises on."""
     if _cuda(k) and all(p.dtype == x.dtype and p.shape[2:] == x.shape[1:] and p.is_contiguous() and x.shape[1] * x.shape[2] * x.element_size() % 16 == 0
                         and x.stride(2) == 1 and x.stride(1) == x.shape[2] and x.stride(0) * x.element_size() % 16 == 0 and x.data_ptr() % 16 == 0 and p.data_ptr() % 16 == 0
                         for p, x in ((k_pool, k), (v_pool, v))):

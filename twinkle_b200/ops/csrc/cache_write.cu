@@ -18,6 +18,7 @@ struct CacheWrite {
   long total, pool_rows;
   int nk, nv;
   long sk, sv;
+  int* err;
 };
 
 __global__ void cache_write_kernel(const CacheWrite p) {
@@ -26,13 +27,17 @@ __global__ void cache_write_kernel(const CacheWrite p) {
     const long t = i / n;
     const int c = static_cast<int>(i - t * n);
     const int64_t row = p.rows[t];
-    if (row < 0 || row >= p.pool_rows) continue;
+    if (row < 0 || row >= p.pool_rows) {        // a block list that names no block of the pool: whoever reads the word next raises
+      atomicCAS(p.err, 0, ERR_BOUNDS);
+      continue;
+    }
     if (c < p.nk) p.kp[row * p.nk + c] = p.k[t * p.sk + c];
     else p.vp[row * p.nv + c - p.nk] = p.v[t * p.sv + c - p.nk];
   }
 }
 
-// pools [blocks, block_size, heads, ·], rows int64 [T] (block · block_size + offset), k and v [T, heads, ·] with heads side by side
+// pools [blocks, block_size, heads, ·], rows int64 [T] (block · block_size + offset), k and v [T, heads, ·] with heads side by side.
+// A row outside the pools is left out and noted in the error word.
 void cache_write(const torch::Tensor& kp, const torch::Tensor& vp, const torch::Tensor& rows, const torch::Tensor& k, const torch::Tensor& v) {
   const int64_t e = k.element_size();
   auto fits = [&](const torch::Tensor& pool, const torch::Tensor& x) {
@@ -55,7 +60,7 @@ void cache_write(const torch::Tensor& kp, const torch::Tensor& vp, const torch::
   p.kp = reinterpret_cast<uint4*>(kp.data_ptr()); p.vp = reinterpret_cast<uint4*>(vp.data_ptr());
   p.rows = rows.data_ptr<int64_t>();
   p.pool_rows = kp.size(0) * kp.size(1);
-  p.sk = k.stride(0) * e / 16; p.sv = v.stride(0) * e / 16;
+  p.sk = k.stride(0) * e / 16; p.sv = v.stride(0) * e / 16; p.err = error_word();
   const int blocks = static_cast<int>(std::min<long>((p.total + 255) / 256, num_sms() * 16L));
   cache_write_kernel<<<blocks, 256, 0, at::cuda::getCurrentCUDAStream()>>>(p);
   count_launch();

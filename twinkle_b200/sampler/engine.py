@@ -478,6 +478,12 @@ class NativeEngine:
                 logits = self.decode_step(nxt, last)
                 live = nxt
         self.release(seqs)
+        if self.device.type == 'cuda':       # before any result leaves: a key that was not stored, a kernel that gave up waiting
+            torch.cuda.current_stream(self.device).synchronize()
+            with torch.cuda.device(self.device):
+                code = ops.ext().read_and_clear_error()
+            if code:
+                raise RuntimeError(f'a kernel reported error {code} during generation (a block outside the cache, or a bounded wait that expired)')
         for s in seqs:
             if not s.params.scoring_only:
                 responses[s.request].sequences.append(SampledSequence(stop_reason=s.stop_reason, tokens=s.tokens, logprobs=s.logprobs,
