@@ -1,5 +1,7 @@
 """GPU numerics of the multi-LoRA, sampler and router kernels against their fp32 PyTorch restatements, plus the
 native sampler and a LoRA training step end to end on the device."""
+import math
+
 import pytest
 import torch
 
@@ -577,3 +579,26 @@ def test_cache_rows_outside_the_pool_are_an_error(E):
     eng._prompt_rows = places
     assert len(eng.generate([[1, 2, 3]], [SamplingParams(max_tokens=2, temperature=0.0)])[0].sequences[0].tokens) == 2
     assert E.read_and_clear_error() == 0
+
+
+def _hashes(seed, n):
+    """The 32-bit hash behind the Gumbel noise of tokens 0 … n of a row."""
+    import numpy as np
+    with np.errstate(over='ignore'):
+        x = np.uint64(seed) * np.uint64(0x9E3779B97F4A7C15) + np.arange(n, dtype=np.uint64)
+        for m in (0xff51afd7ed558ccd, 0xc4ceb9fe1a85ec53):
+            x = (x ^ (x >> np.uint64(33))) * np.uint64(m)
+        return (x ^ (x >> np.uint64(33))).astype(np.uint32)
+
+
+def test_sampling_hash_that_rounds_to_one(E):
+    """A token whose uniform number rounds to 1 gets a large but finite score: it loses to tokens of e^30 times its weight, and wins among equals."""
+    from twinkle_b200 import ops
+    V = 151936
+    seed, at = next((s, int(h.argmax())) for s, h in ((s, _hashes(s, V)) for s in range(4000)) if h.max() >= 2**32 - 128)
+    x = torch.zeros(1, V, device='cuda')
+    seeds = torch.tensor([seed], device='cuda')
+    assert int(ops.sample_tokens(x, 1.0, -1, 1.0, seeds=seeds)[0]) == at          # ln 2^26 = 18 of the others' 12 at most, as a rule
+    x[0, at] = -30.0
+    tok, lp = ops.sample_tokens(x, 1.0, -1, 1.0, seeds=seeds)
+    assert int(tok) != at and abs(float(lp) + math.log(V)) < 1e-4

@@ -304,7 +304,10 @@ sample_kernel(const float* __restrict__ logits, const int64_t* __restrict__ seed
       }
       if (__any_sync(0xffffffffu, open)) {
         if (open) {
-          const float score = p.x[i] * inv_temp - __logf(-__logf(u));
+          // Hashes from 2^32 − 128 on round to u = 1, where E = 0 would let a token win whatever its logit (one row in 220 at 152 k tokens); they
+          // stand for 1 − u = 2^-26 on average.
+          const float E = u < 1.f ? -__logf(u) : 0x1p-26f;
+          const float score = p.x[i] * inv_temp - __logf(E);
           if (score > best) { best = score; best_i = begin + i; }
         }
         bar = 0.999f * __expf(warp_max(best) - p.mx);
