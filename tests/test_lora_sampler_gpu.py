@@ -602,3 +602,83 @@ def test_sampling_hash_that_rounds_to_one(E):
     x[0, at] = -30.0
     tok, lp = ops.sample_tokens(x, 1.0, -1, 1.0, seeds=seeds)
     assert int(tok) != at and abs(float(lp) + math.log(V)) < 1e-4
+
+
+def test_sampling_leaves_out_no_winner_near_one(E):
+    """Two tokens of one warp with u within 2^-17 of 1, where the error of the fast logarithm makes e / E larger than the exact bound e / (1 − u): the later one
+    wins by a little, and must not be passed over because of the earlier one."""
+    import numpy as np
+
+    from twinkle_b200 import ops
+    V, found = 8192, []
+    for seed in range(60000):
+        h = _hashes(seed, V)
+        near = np.nonzero(h >= 2**32 - 200 * 256)[0]
+        for a in near:
+            for b in near:
+                # steps of 2^-24 below 1; the same warp (512 threads per round), a later round
+                ka, kb = (2**24 - int(np.float32(h[i]) / 256) for i in (a, b))
+                if b // 512 > a // 512 and b % 512 // 32 == a % 512 // 32 and kb >= 2 * ka and ka >= 8:
+                    found.append((seed, int(a), int(b), ka, kb))
+        if len(found) >= 2:
+            break
+    assert len(found) >= 2
+    for seed, a, b, ka, kb in found:
+        # e_b / e_a between E_b / E_a as the exact logarithm has it and 0.999 (1 − u_b) / E_a with the fast one's E_a, about 0.8 steps less
+        ratio = kb / (ka - 0.8) * (1 - 0.4 / kb)
+        x = torch.full((1, V), -100.0, device='cuda')
+        x[0, a], x[0, b] = 0.0, math.log(ratio)
+        assert int(ops.sample_tokens(x, 1.0, -1, 1.0, seeds=torch.tensor([seed], device='cuda'))[0]) == b, (seed, a, b, ka, kb)
+
+
+@pytest.mark.parametrize('V', [32, 1000, 8192, 20001, 60000, 151936, 400001])
+@pytest.mark.parametrize('rows', [3, 300])
+@pytest.mark.parametrize('how', [(1.0, -1, 1.0), (0.7, 50, 1.0), (1.0, -1, 0.9)])
+def test_sampling_draws_the_largest_score(E, V, rows, how):
+    """The drawn token has the largest of logit / T + Gumbel noise among those kept, recomputed in fp64 from the hash, for one to eight CTAs per row, in shared
+    memory and beyond it.  Scores are uncertain by what __logf leaves: 2^-21 of E = −ln u."""
+    import numpy as np
+
+    from twinkle_b200 import ops
+    if rows == 300 and V > 200000:
+        rows = 40
+    temp, k, p = how
+    g = torch.Generator(device='cuda').manual_seed(V + rows)
+    x = torch.randn(rows, V, device='cuda', generator=g) * 2
+    seeds = torch.arange(rows, device='cuda') * 7919 + V
+    tok, _ = ops.sample_tokens(x, temp, k, p, seeds=seeds)
+    some = sorted(set(range(0, rows, max(1, rows // 12))))
+    wins = 0
+    for r in some:
+        h = torch.from_numpy(_hashes(int(seeds[r]), V).astype(np.int64)).cuda()
+        u = (h.float() + 0.5) * 2.0 ** -32
+        en = torch.where(u < 1, -torch.log(u.double()), 2.0 ** -26)
+        blur = torch.where(u < 1, -torch.log1p(-(2.0 ** -21 / en).clamp_max(1 - 1e-9)), 0) + 1e-4
+        prob = torch.softmax(x[r].double() / temp, -1)
+        top = prob.sort(descending=True)[0]
+        tau = top[k - 1] if 0 < k < V else top[(top.cumsum(-1) < p).sum().clamp_max(V - 1)] if p < 1 else torch.zeros((), device='cuda', dtype=torch.float64)
+        score = x[r].double() / temp - torch.log(en)
+        sure = (prob >= tau * (1 + 1e-4) + top[0] * 2.0 ** -31) | (prob == top[0])
+        t = int(tok[r])
+        assert prob[t] >= tau * (1 - 1e-4) - top[0] * 2.0 ** -31
+        assert float(score[t] + blur[t]) >= float((score - blur)[sure].max()), r
+        wins += t == int(torch.where(sure, score, -torch.inf).argmax())
+    assert wins >= len(some) - 1          # the blur decides next to nothing
+    # a row is cut differently in a batch and alone
+    one = torch.cat([ops.sample_tokens(x[r:r + 1], temp, -1, 1.0, seeds=seeds[r:r + 1])[0] for r in some])
+    assert torch.equal(one, ops.sample_tokens(x, temp, -1, 1.0, seeds=seeds)[0][some])
+
+
+def test_sampling_frequencies_over_a_wide_row(E):
+    """Tokens in every CTA of a cluster and many per lane: drawn as often as their probabilities say."""
+    from twinkle_b200 import ops
+    V, n = 151936, 20000
+    live = torch.linspace(3, V - 5, 24, device='cuda').long()
+    weight = torch.arange(1, 25, device='cuda').double()
+    x = torch.full((V, ), -60.0, device='cuda')
+    x[live] = weight.log().float()
+    got = torch.cat([ops.sample_tokens(x.expand(500, V).contiguous(), 1.0, -1, 0.999, seeds=torch.arange(i, i + 500, device='cuda'))[0] for i in range(0, n, 500)])
+    count = (got[:, None] == live).sum(0).double()
+    want = weight / weight.sum() * n
+    assert int(count.sum()) == n
+    assert float(((count - want) ** 2 / want).sum()) < 23 + 5 * (2 * 23) ** 0.5         # chi-squared of 23 degrees: mean 23, variance 46

@@ -292,15 +292,17 @@ sample_kernel(const float* __restrict__ logits, const int64_t* __restrict__ seed
     }
   } else {
     // With E = −ln u the score is ln(e / E) + max, and E ≥ 1 − u: an element with e / (1 − u) well below what the warp has already cannot win, and
-    // its logarithms are not taken (64 x 151936 without a search: 89 → 71 us, at the occupancy of one CTA per SM).
-    float bar = -1.f;                 // the warp's best e / E, a little less
+    // its logarithms are not taken (64 x 151936 without a search: 89 → 71 us, at the occupancy of one CTA per SM).  Near u = 1 the error of __logf is
+    // absolute, up to 2^-21.41 by its documentation, so what is compared is (1 − u) − 2^-21; the 0.1 % is for the relative errors of e, of logarithms elsewhere
+    // and of scores, whose magnitude is taken to stay below 2^12.  Then nothing that would win is left out, however the row is cut.
+    float bar = 0.f;                  // the warp's best e / E, a little less
     for (int i = threadIdx.x; i - static_cast<int>(threadIdx.x & 31) < p.n; i += THREADS) {
       bool open = false;
       float u = 0.f;
       if (i < p.n) {
         const float e = p.at(i);
         u = (static_cast<float>(mix32(seed * 0x9E3779B97F4A7C15ull + static_cast<uint64_t>(begin + i))) + 0.5f) * (1.f / 4294967296.f);
-        open = !(e < tau) && !(e < bar * (1.f - u));
+        open = !(e < tau) && !(e < fmaf(-bar, u, bar * (1.f - 0x1p-21f)));
       }
       if (__any_sync(0xffffffffu, open)) {
         if (open) {
