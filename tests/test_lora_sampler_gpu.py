@@ -682,3 +682,22 @@ def test_sampling_frequencies_over_a_wide_row(E):
     want = weight / weight.sum() * n
     assert int(count.sum()) == n
     assert float(((count - want) ** 2 / want).sum()) < 23 + 5 * (2 * 23) ** 0.5         # chi-squared of 23 degrees: mean 23, variance 46
+
+
+@pytest.mark.parametrize('hq,hkv,d', [(32, 8, 128), (16, 4, 64), (16, 8, 128)])
+@pytest.mark.parametrize('n', [5, 100, 1500])
+def test_paged_decode_of_infinite_values(E, hq, hkv, d, n):
+    """An infinite value among the visible ones is the result in its dimension, of either sign; two of opposite signs make NaN; other dimensions are as without it."""
+    from twinkle_b200 import ops
+    g = torch.Generator(device='cuda').manual_seed(n)
+    blocks = (n + 15) // 16 + 1
+    kc, vc = (torch.randn(blocks, 16, hkv, d, device='cuda', generator=g).bfloat16() for _ in range(2))
+    q = torch.randn(1, hq, d, device='cuda', generator=g).bfloat16()
+    table, lens = torch.arange(blocks, device='cuda').int()[None], torch.tensor([n], device='cuda').int()
+    plain = ops.paged_attention_decode(q, kc, vc, table, lens)
+    rows, last = vc.view(-1, hkv, d), blocks * 16 - 1
+    rows[n // 2, :, 3], rows[n - 1, :, 10], rows[0, :, 20], rows[n - 1, :, 20], rows[last, :, 30] = math.inf, -math.inf, math.inf, -math.inf, math.nan
+    o = ops.paged_attention_decode(q, kc, vc, table, lens)
+    assert (o[..., 3] == math.inf).all() and (o[..., 10] == -math.inf).all() and o[..., 20].isnan().all()
+    rest = [i for i in range(d) if i not in (3, 10, 20)]
+    assert torch.equal(o[..., rest], plain[..., rest])
