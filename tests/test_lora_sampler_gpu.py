@@ -701,3 +701,24 @@ def test_paged_decode_of_infinite_values(E, hq, hkv, d, n):
     assert (o[..., 3] == math.inf).all() and (o[..., 10] == -math.inf).all() and o[..., 20].isnan().all()
     rest = [i for i in range(d) if i not in (3, 10, 20)]
     assert torch.equal(o[..., rest], plain[..., rest])
+
+
+@pytest.mark.parametrize('window,chunk,at', [(70, 0, 200), (1, 0, 300), (0, 128, 300), (0, 384, 383), (130, 0, 120)])
+@pytest.mark.parametrize('d,e', [(128, 128), (64, 40)])
+@pytest.mark.parametrize('lens', [(512, ), (300, 509)])
+def test_flash_forward_values_before_a_tile(E, window, chunk, at, d, e, lens):
+    """Values that are not finite in a key block before everything that a query tile sees leave its rows as they are, also when the tile's neighbour sees the block."""
+    g = torch.Generator(device='cuda').manual_seed(at)
+    T, n = sum(lens), lens[-1]
+    q, k, v = (torch.randn(T, h, w, device='cuda', generator=g).bfloat16() for h, w in ((6, d), (2, d), (2, e)))
+    cu = torch.tensor([0] + list(lens), device='cuda').cumsum(0).int()
+    run = lambda v: E.flash_attn_fwd(q, k, v, cu, max(lens), True, d ** -0.5, None, None, None, window, chunk)  # noqa: E731
+    plain, lse = run(v)
+    bad = v.clone()
+    bad[T - n + at, :, 0], bad[T - n + at, :, 1] = math.inf, math.nan
+    o, lse2 = run(bad)
+    tile = next(t for t in range(0, n, 128) if (t - window + 1 if window else t // chunk * chunk) // 128 > at // 128)       # the first that sees later blocks only
+    assert torch.equal(o[T - n + tile:], plain[T - n + tile:]) and torch.equal(lse, lse2)
+    seen = slice(T - n + at, T - n + at + 1)
+    assert (o[seen, :, 0] == math.inf).all() and o[seen, :, 1].isnan().all()
+    assert E.read_and_clear_error() == 0

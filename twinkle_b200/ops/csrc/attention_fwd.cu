@@ -431,6 +431,8 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   auto end_of = [&](int t) { return q0 + t * BQ >= seq_len ? 0 : p.causal ? max(0, min(kv_len, q0 + (t + 1) * BQ + q_off)) : kv_len; };
   auto blocks_of = [&](int t) { return max(0, (end_of(t) + BKV - 1) / BKV - jb0); };
   const int n_a = blocks_of(0), n_b = blocks_of(1), n_all = max(n_a, n_b);
+  // the second tile leaves out blocks before all of its rows' bounds, as a tile of its own would: a weight of zero does not cancel a value that is not finite
+  const int begin_b = bounded ? first_visible(max(q0 + BQ + q_off, 0), p.window, p.chunk) / BKV - jb0 : 0;
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -521,7 +523,7 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     if (ok) {
       tc_fence_after();
       if (n_a > 0) scores(0, 0);
-      if (n_b > 0) scores(1, 0);
+      if (n_b > 0 && begin_b == 0) scores(1, 0);
       commit(&k_empty[0]);
     }
     for (int j = 0; ok && j < n_all; ++j) {
@@ -530,26 +532,27 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       if (j + 1 < n_all && !wait(&k_full[(j + 1) & 1], ((j + 1) >> 1) & 1)) break;
 #pragma unroll 1
       for (int t = 0; t < 2; ++t) {
-        const int n = t == 0 ? n_a : n_b;
-        if (j >= n) continue;
-        ok = wait(&p_ready[t], j & 1);
-        if (!ok) break;
-        tc_fence_after();
-        if (elect_one()) {
+        const int n = t == 0 ? n_a : n_b, begin = t == 0 ? 0 : begin_b;
+        if (j >= begin && j < n) {
+          ok = wait(&p_ready[t], (j - begin) & 1);
+          if (!ok) break;
+          tc_fence_after();
+          if (elect_one()) {
 #pragma unroll
-          for (int k = 0; k < BKV / 16; ++k)
-            umma_bf16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + k * 8, dv + k * (2048 >> 4), idesc_o, k > 0 ? 1u : static_cast<uint32_t>(j > 0));
-          if (j == n - 1) umma_commit(&o_done[t]);
+            for (int k = 0; k < BKV / 16; ++k)
+              umma_bf16_ts(tmem_base + 256 + t * 128, tmem_base + t * 128 + k * 8, dv + k * (2048 >> 4), idesc_o, k > 0 ? 1u : static_cast<uint32_t>(j > begin));
+            if (j == n - 1) umma_commit(&o_done[t]);
+          }
+          __syncwarp();
         }
-        __syncwarp();
-        if (j + 1 < n) scores(t, j + 1);                 // runs after the product that reads P from the same columns
+        if (j + 1 >= begin && j + 1 < n) scores(t, j + 1);     // runs after the product that reads P from the same columns
       }
       commit(&v_empty[j & 1]);
       if (j + 1 < n_all) commit(&k_empty[(j + 1) & 1]);
     }
   } else {
     // -------------------------------------------------------------- softmax
-    const int t = warp >> 2, qt = q0 + t * BQ, n_blocks = t == 0 ? n_a : n_b, kv_end = end_of(t);
+    const int t = warp >> 2, qt = q0 + t * BQ, begin = t == 0 ? 0 : begin_b, n_blocks = t == 0 ? n_a : n_b, kv_end = end_of(t);
     const int row = (warp & 3) * 32 + lane, q_pos = qt + row;
     const uint32_t lane_off = static_cast<uint32_t>((warp & 3) * 32) << 16;
     const uint32_t ts = tmem_base + t * 128 + lane_off, to = tmem_base + 256 + t * 128 + lane_off;
@@ -559,8 +562,8 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     float m_used = -INFINITY;
     float2 l2 = make_float2(0.f, 0.f);       // sums over the first and second 64 keys of the blocks
     bool dead = false;
-    for (int j = 0; j < n_blocks; ++j) {
-      if (!mbar_wait(&s_full[t], j & 1, p.err, ERR_ATTN_WAIT)) { dead = true; break; }
+    for (int j = begin; j < n_blocks; ++j) {
+      if (!mbar_wait(&s_full[t], (j - begin) & 1, p.err, ERR_ATTN_WAIT)) { dead = true; break; }
       tc_fence_after();
       float sc[128];
 #pragma unroll
@@ -593,7 +596,7 @@ flash_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       // a row may see none of its first blocks: its maximum then stays at −∞ and its weights are zero
       if (mx > m_used + RESCALE_THRESHOLD || (m_used == -INFINITY && mx != -INFINITY)) {
         alpha = (m_used == -INFINITY) ? 0.f : exp2f(m_used - mx);
-        rescale = (j > 0);
+        rescale = (j > begin);
         m_used = mx;
         l2.x *= alpha;
         l2.y *= alpha;
