@@ -722,3 +722,10 @@ def test_flash_forward_values_before_a_tile(E, window, chunk, at, d, e, lens):
     seen = slice(T - n + at, T - n + at + 1)
     assert (o[seen, :, 0] == math.inf).all() and o[seen, :, 1].isnan().all()
     assert E.read_and_clear_error() == 0
+
+
+@pytest.mark.parametrize('H', [256, 768, 1536, 2560, 3072, 3584, 4864, 5120, 5376])
+@pytest.mark.parametrize('rows', [1, 149, 2400])
+def test_rmsnorm_of_any_multiple_of_256(E, H, rows):
+    """Every width whose rows fit registers, and the first beyond them."""
+    test_rmsnorm_rows_in_registers(E, H, rows)

@@ -68,8 +68,10 @@ __global__ void rmsnorm_fwd_kernel(const bf16* __restrict__ x, const bf16* __res
   }
 }
 
-// The same for rows of NV·256 elements, which fit a warp's registers: every load of a row is on its way at once and the row is read once.
-// 64 x 4096 14.2 → 3.3 us (4.8 with a residual), 1 x 1024 4.4 → 2.1 (2.5): the latency of one load instead of two chains.
+// The same for rows of NV·256 elements, up to 5120, which fit a warp's registers: every load of a row is on its way at once and the row is read once, in
+// the same order of sums.  The width is a constant of the kernel: with a count of vectors at run time the loads wait for one another (64 x 4096: 5.5 us against
+// 2.5).  us before → now without and with a residual: 64 x 1024 2.9, 3.5 → 1.8, 2.0; 64 x 3072 5.8, 7.4 → 2.3, 2.8; 64 x 4096 7.2, 9.1 → 2.5, 3.2; 64 x 5120 8.6, 10.6 → 2.7,
+// 4.2; 16384 x 2048 26.9, 48.1 → 23.7, 44; 16384 x 3072 39.9, 75.4 → 40.0, 63.4; 16384 x 5120 77, 136 → 66, 114; nothing slower from 1 x 256 to 16384 x 5120.
 template <int NV, bool RES>
 __global__ void rmsnorm_fwd_regs_kernel(const bf16* __restrict__ x, const bf16* __restrict__ res, const bf16* __restrict__ w, bf16* __restrict__ y, bf16* __restrict__ hsum,
                                         float* __restrict__ rstd, int rows, float eps, float offset) {
@@ -291,6 +293,13 @@ __global__ void rmsnorm_bwd_kernel(const bf16* __restrict__ g, const bf16* __res
   }
 }
 
+// f(NV) for the one of 1 … MOST with H = NV·256; false where there is none.
+template <int MOST, typename F>
+static bool for_width(int H, F&& f) {
+  if (H == MOST * 256) return f(std::integral_constant<int, MOST>{}), true;
+  if constexpr (MOST > 1) return for_width<MOST - 1>(H, f); else return false;
+}
+
 // Returns {y, rstd} or, with a residual, {y, rstd, h} where h = x + residual is the row that was normalised.
 std::vector<torch::Tensor> rmsnorm_fwd(const torch::Tensor& x, const torch::Tensor& w, double eps, double offset,
                                        const c10::optional<torch::Tensor>& residual) {
@@ -314,10 +323,11 @@ std::vector<torch::Tensor> rmsnorm_fwd(const torch::Tensor& x, const torch::Tens
           reinterpret_cast<bf16*>(y.data_ptr()), has_res ? reinterpret_cast<bf16*>(h.data_ptr()) : nullptr, rstd.data_ptr<float>(), rows, static_cast<float>(eps),
           static_cast<float>(offset));
     };
-    if (H == 1024) { if (has_res) regs(rmsnorm_fwd_regs_kernel<4, true>); else regs(rmsnorm_fwd_regs_kernel<4, false>); }
-    else if (H == 2048) { if (has_res) regs(rmsnorm_fwd_regs_kernel<8, true>); else regs(rmsnorm_fwd_regs_kernel<8, false>); }
-    else if (H == 4096) { if (has_res) regs(rmsnorm_fwd_regs_kernel<16, true>); else regs(rmsnorm_fwd_regs_kernel<16, false>); }
-    else {
+    const bool in_registers = for_width<20>(H, [&](auto nv) {
+      constexpr int NV = decltype(nv)::value;
+      if (has_res) regs(rmsnorm_fwd_regs_kernel<NV, true>); else regs(rmsnorm_fwd_regs_kernel<NV, false>);
+    });
+    if (!in_registers) {
       int blocks = std::min((rows + 7) / 8, num_sms() * 8);
       rmsnorm_fwd_kernel<<<blocks, 256, 0, at::cuda::getCurrentCUDAStream()>>>(
           reinterpret_cast<const bf16*>(x.data_ptr()), has_res ? reinterpret_cast<const bf16*>(residual->data_ptr()) : nullptr,
