@@ -84,15 +84,6 @@ class PagedKVCache:
     def blocks_for(self, n_tokens: int) -> int:
         return (n_tokens + self.block_size - 1) // self.block_size
 
-    def write(self, layer: int, blocks: Sequence[int], start: int, k: torch.Tensor, v: torch.Tensor) -> None:
-        """Store ``k, v [n, Hkv, D]`` at token positions ``start .. start+n`` of a sequence."""
-        n = k.shape[0]
-        pos = torch.arange(start, start + n, device=k.device)
-        blk = torch.as_tensor(blocks, device=k.device)[pos // self.block_size]
-        off = pos % self.block_size
-        self.k[layer][blk, off] = k
-        self.v[layer][blk, off] = v
-
 
 @dataclass
 class _Seq:
