@@ -206,8 +206,10 @@ static void launch_paged_decode(const torch::Tensor& q, const torch::Tensor& kc,
         reinterpret_cast<const T*>(vc.data_ptr()), tables.data_ptr<int>(), seq_lens.data_ptr<int>(), reinterpret_cast<T*>(out.data_ptr()), hq, hkv, d, e,
         static_cast<int>(kc.size(1)), static_cast<int>(tables.size(1)), sl2, G, extras);
   };
-  // Where the CTAs leave SMs idle a head has one of its own: a step is bound by the instructions of a warp per token, not by the rows that two CTAs
-  // then read (one sequence of 1 k tokens, 16/8 heads of 128: 20.6 → 19.3 us), and every head is computed as before.
+  // Where the CTAs leave SMs idle a head has one of its own: a step is bound by the instructions of a warp per token, not by the rows that several CTAs
+  // then read.  Up to two heads per SM, us with heads together → alone, caches larger than L2 in turn: bf16 16/8 heads of 128, 1 sequence of 1 k tokens 36.2 → 34.2,
+  // 16 of 8 k (256 heads) 272 → 274; 12/4 39.2 → 30.8, 304 → 247 (192 heads); with score terms 32/8 50 → 33, 388 → 281 (256 heads); heads of 256, 8/4 61.3 → 61.0, 469 → 458; fp32
+  // 32/4 50.7 → 49.1, 384 → 375.  Sums keep their order; the compiler may contract multiply-adds of the two forms differently (last bits).
   const bool alone = static_cast<long>(B) * hq <= 2 * num_sms();
   const int vectors = (std::max(d, e) + 8 * V - 1) / (8 * V);   // per lane
   if (vectors <= 1) {

@@ -4,7 +4,8 @@
 // rows.  Here a CTA takes one 128-row tile of x (only its live rows are loaded) and BN weight rows, BN any multiple of 16, and a cluster of S CTAs
 // may share a tile by parts of K, added up in rank order through distributed shared memory.  A stage is one TMA load of x and one of W, each KA
 // 64-wide swizzle atoms deep (a 3-D map {64, rows, K/64}), the stages fill shared memory, and one tile per CTA leaves nothing to schedule.
-// Products run over K in the same steps of 16 as in gemm.cu, so results without a split are the same to the bit.
+// Products run over K in the same steps of 16 as in gemm.cu, so results without a split are the same to the bit; a split in two, which follows the number of rows, halves
+// the distance from 64 bits (K = 12288: 1.4e-5 → 6.8e-6).
 //
 // What bounds it: memory for wide weights (1 x 24576 x 4096: 53 → 36 us at a floor of 31), the issue of products, 35 ns each, for small ones.
 // us before → now: 64 rows, N x K 6144 x 4096 30 → 16, 4096 x 4096 29 → 14, 4096 x 12288 76 → 26, 24576 x 4096 53 → 38; 1 row, 1024 x 3072
@@ -195,8 +196,9 @@ __global__ void __launch_bounds__(gs::THREADS) gemm_skinny_kernel(const __grid_c
   }
 }
 
-// Few rows: up to one tile of them whatever the width (64 x 24576 x 4096: 38 us, 53 in pair tiles), and beyond that where neither kind of larger tile
-// occupies half of the chip (256 x 4096 x 4096: 16 us, 30 in 128x256 tiles; 256 x 24576 x 4096: 63, 54 in pair tiles).
+// Few rows: up to one tile of them whatever the width (64 x 24576 x 4096: 38 us, 53 in pair tiles), and beyond that where pair tiles would occupy less than the
+// chip, or 128x256 tiles less than one wave of it (256 x 4096 x 4096: 16 us, 30 in 128x256 tiles).  At the line both are equal (1024 rows, N x K 4096 x 1024 12.8 us against 13.1, 4096 x
+// 4096 31.0 and 31.5, 4096 x 12288 81.0 and 79.1); beyond it wide tiles win (256 x 24576 x 4096: 63 us, 54 in pair tiles).
 static bool is_skinny(int M, int N) {
   return M <= 128 || std::min(static_cast<long>((M + 255) / 256) * ((N + 255) / 256), static_cast<long>((M + 127) / 128) * ((N + 255) / 256) / 2) < num_sms() / 2;
 }

@@ -251,9 +251,9 @@ static void launch(const PagedDecode& p, int B, cudaStream_t stream) {
 bool paged_decode_mma(const PagedDecode& p, int B, int d, int e, cudaStream_t stream) {
   // cp.async and the query's pairs want the pools on 16-byte and the query on 4-byte boundaries
   const bool aligned = reinterpret_cast<uintptr_t>(p.kc) % 16 == 0 && reinterpret_cast<uintptr_t>(p.vc) % 16 == 0 && reinterpret_cast<uintptr_t>(p.q) % 4 == 0;
-  // Groups of one to three heads stay with the vector kernel: it has a quarter to three quarters of the arithmetic per byte there, and decoders
-  // that have such groups are small and deep, where sums in another order move the logits of a 28-layer stack by 3 % (every layer's rounding
-  // to bf16 falls differently), as much as bf16 itself.
+  // Groups of one to three heads stay with the vector kernel, which is the slower one there (16/8 heads, one sequence of 1 k tokens: 19.3 us against 6.3): the
+  // decoders that have such groups are small and deep, and any other order of these sums moves the logits of a 28-layer stack by 2.7–3.8 %, at the same
+  // distance from 64 bits (3.7–4.1 %).  perf/cases.py grants such stacks 3 %, so their steps keep the order that they had.
   if (!aligned || p.G < 4 || d != e || (d != 64 && d != 128) || B > 65535 || p.hkv * ((p.G + pd::HEADS - 1) / pd::HEADS) > 65535) return false;
   if (d == 64) launch<64>(p, B, stream); else launch<128>(p, B, stream);
   return true;

@@ -35,7 +35,6 @@ struct SampleShared {
   float all[sm::NT + 1];
   int idx[sm::WARPS], best_i;
   int overflow;
-  int list_n[sm::WARPS];
 };
 
 // Sums (or the maximum) of N values over the cluster, the same bits in every thread.
